@@ -438,6 +438,7 @@ int general_status(kmsd_batch_s *bt, cudaStream_t s) {
             default: return fail(KMSD_EMETRIC, "S solve failed true-residual acceptance");
         }
     }
+    if (st[3] != 0) return fail(KMSD_ERUNTIME, "a bounded device wait ran out");
     return KMSD_OK;
 }
 

@@ -454,7 +454,11 @@ int kmsd_csr_create(int64_t n, const int64_t *indptr, const int64_t *indices, co
             if (!rc) rc = up((void **)&A->bsr_idx, bcols.data(), nblk * sizeof(int));
             if (!rc) rc = up((void **)&A->bsr_re, br.data(), br.size() * sizeof(double));
             if (!rc && cplx) rc = up((void **)&A->bsr_im, bi.data(), bi.size() * sizeof(double));
-            if (!rc) A->bsr_nb = nbr;
+            if (!rc) {
+                A->bsr_nb = nbr;
+                A->bsr_ptr_host.swap(bptr);
+                A->bsr_idx_host.swap(bcols);
+            }
         }
     }
     if (rc) {

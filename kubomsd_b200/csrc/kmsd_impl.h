@@ -82,6 +82,7 @@ struct kmsd_csr_s {
     int64_t bsr_nb = 0;
     int *bsr_ptr = nullptr, *bsr_idx = nullptr;
     double *bsr_re = nullptr, *bsr_im = nullptr;
+    std::vector<int> bsr_ptr_host, bsr_idx_host;  // the block pattern (halos of the resident solve)
     int ensure_f32();
     kmsd::CsrView<double> view64() const { return {ptr, idx, re64, complex_values ? im64 : nullptr}; }
     kmsd::CsrView<float> view32() const { return {ptr, idx, re32, complex_values ? im32 : nullptr}; }
@@ -142,6 +143,15 @@ struct kmsd_metric_s {
     kmsd::DevBuf q, y, r, z, p, sp, t;
     kmsd::DevBuf cols;       // per-column state (PcgCols layout)
     kmsd::DevBuf host_pinned;  // pinned host flags
+    // Resident solve (kmsd_pcg.cu): meeting counter and packets of partial
+    // sums; per CTA count, the block columns that each CTA's rows touch.
+    kmsd::DevBuf resident;
+    struct Halo {
+        kmsd::DevBuf mem;
+        int *off = nullptr, *list = nullptr, *local = nullptr, *self = nullptr;
+        int own = 0, blocks = 0, most = 0;  // of the largest CTA share
+    };
+    std::map<int, Halo> halos;
     kmsd::Reducer red;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     // counters (host side, plus device counters folded in on read)

@@ -11,6 +11,11 @@
 // live on the device and are updated by the last CTA of each reduction
 // kernel, so an iteration needs no host round trip.  The host polls a single
 // halt word once per chunk of iterations to stop launching.
+//
+// A single system of 4x4 blocks whose shares fit shared memory is solved by one
+// launch instead (kmsd_pcg.cu); the launch sequence here serves CSR overlaps,
+// other block sizes, segmented solves, complex64 work vectors and systems too
+// large for that.
 #include <math.h>
 #include <float.h>
 #include <algorithm>
@@ -24,48 +29,11 @@
 #include "kmsd.h"
 #include "kmsd_impl.h"
 #include "kmsd_kernels.cuh"
+#include "kmsd_pcg.cuh"
 
 using namespace kmsd;
 
 namespace {
-
-struct ColPtr {
-    double *safe, *bn, *thr, *rz, *alpha, *beta, *rn, *tn, *newrz, *gap, *relative, *residual;
-    double *rsn;  // residual norm at the last (re)start (mixed form)
-    int *active, *restart, *brk, *conv, *finp, *fino;
-    long long *iters;
-    int *flags;  // [0] halt, [1] check, [2] nonfinite rhs, [3] breakdown, [4] n_active
-};
-constexpr int kDoubles = 13, kInts = 6;
-size_t col_bytes(int64_t b) { return (size_t)b * (kDoubles * 8 + kInts * 4 + 8) + 64; }
-ColPtr col_ptr(void *base, int64_t b) {
-    ColPtr c;
-    double *d = static_cast<double *>(base);
-    double **dp[kDoubles] = {&c.safe, &c.bn, &c.thr, &c.rz, &c.alpha, &c.beta,       &c.rn,
-                             &c.tn,   &c.newrz, &c.gap, &c.relative, &c.residual, &c.rsn};
-    for (int i = 0; i < kDoubles; ++i) *dp[i] = d + (size_t)i * b;
-    long long *l = reinterpret_cast<long long *>(d + (size_t)kDoubles * b);
-    c.iters = l;
-    int *ip = reinterpret_cast<int *>(l + b);
-    int **ipp[kInts] = {&c.active, &c.restart, &c.brk, &c.conv, &c.finp, &c.fino};
-    for (int i = 0; i < kInts; ++i) *ipp[i] = ip + (size_t)i * b;
-    c.flags = ip + (size_t)kInts * b;
-    return c;
-}
-// device counters: [0] refreshes [1] checks [2] restarts [3] iterations sum; [4] max relative (double bits)
-struct Counters {
-    long long v[4];
-    double max_rel;
-};
-
-struct Pre {
-    const double *diag;
-    const int *bstart;
-    const int64_t *foff;
-    const double2 *factors;
-    int ub;    // uniform block size, or 0: rows and factors are then found without lookups
-    int real;  // every block inverse is real
-};
 
 __device__ __forceinline__ double2 cdiv(double2 a, double2 b) {
     if (fabs(b.x) >= fabs(b.y)) {
@@ -1401,58 +1369,54 @@ int kmsd_metric_s::solve(const double2 *B, double2 *Y, int64_t b, double rtol, d
     PcgFn fn = pick(mu_for(mp), nblocks ? maxb : 1, sf, seg, store32 != 0);
     if (!fn) return fail(KMSD_EINVAL, "unsupported metric block size / column count");
     const bool sync = status == nullptr;
+    ResidentPlan plan;
+    if (int rc = resident_plan(this, b, &plan)) return rc;
     // Synchronous calls use a private status word and report.
     static thread_local DevBuf own_status, own_report;
     int *st = status;
     FailReportFull *fr = static_cast<FailReportFull *>(fail_report);
     int *claimed = nullptr;
     if (sync) {
-        if (own_status.ensure(2 * sizeof(int))) return KMSD_ECUDA;
+        if (own_status.ensure(4 * sizeof(int))) return KMSD_ECUDA;
         if (own_report.ensure(sizeof(FailReportFull))) return KMSD_ECUDA;
         st = own_status.as<int>();
         fr = own_report.as<FailReportFull>();
-        KMSD_CUDA(cudaMemsetAsync(st, 0, 2 * sizeof(int), s));
+        KMSD_CUDA(cudaMemsetAsync(st, 0, 4 * sizeof(int), s));
     }
     claimed = st + 1;
-    int rc = fn(this, B, Y, b, rtol, atol, maxiter, s, st, fr, claimed, kHostLoop);
+    int rc = plan.form ? resident_solve(this, plan, B, Y, b, rtol, atol, maxiter, s, st, fr)
+                       : fn(this, B, Y, b, rtol, atol, maxiter, s, st, fr, claimed, kHostLoop);
     if (rc) return rc;
     ++calls;
     if (!sync) return KMSD_OK;
-    // Read status + per-column report (segment-major for a segmented solve).
-    ColPtr c = col_ptr(cols.p, ncols);
-    std::vector<int> conv(ncols), brk(ncols), flags(8);
-    std::vector<long long> it(ncols);
-    std::vector<double> res(ncols), rel(ncols);
-    int hst[2];
-    KMSD_CUDA(cudaMemcpyAsync(conv.data(), c.conv, ncols * sizeof(int), cudaMemcpyDeviceToHost, s));
-    KMSD_CUDA(cudaMemcpyAsync(brk.data(), c.brk, ncols * sizeof(int), cudaMemcpyDeviceToHost, s));
-    KMSD_CUDA(cudaMemcpyAsync(it.data(), c.iters, ncols * sizeof(long long), cudaMemcpyDeviceToHost, s));
-    KMSD_CUDA(cudaMemcpyAsync(res.data(), c.residual, ncols * sizeof(double), cudaMemcpyDeviceToHost, s));
-    KMSD_CUDA(cudaMemcpyAsync(rel.data(), c.relative, ncols * sizeof(double), cudaMemcpyDeviceToHost, s));
-    KMSD_CUDA(cudaMemcpyAsync(flags.data(), c.flags, 8 * sizeof(int), cudaMemcpyDeviceToHost, s));
-    KMSD_CUDA(cudaMemcpyAsync(hst, st, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+    // Read the status and the column state (segment-major for a segmented
+    // solve), which is one allocation, in one copy.
+    std::vector<unsigned char> host(col_bytes(ncols));
+    const ColPtr h = col_ptr(host.data(), ncols);
+    int hst[4];
+    KMSD_CUDA(cudaMemcpyAsync(host.data(), cols.p, host.size(), cudaMemcpyDeviceToHost, s));
+    KMSD_CUDA(cudaMemcpyAsync(hst, st, sizeof(hst), cudaMemcpyDeviceToHost, s));
     KMSD_CUDA(cudaStreamSynchronize(s));
     seconds += std::chrono::duration<double>(std::chrono::steady_clock::now() - start).count();
+    if (hst[3]) return fail(KMSD_ERUNTIME, "a bounded device wait of the metric solve ran out");
     if (report) {
         for (int64_t j = 0; j < ncols; ++j) {
-            report->converged[j] = (uint8_t)conv[j];
-            report->breakdown[j] = (uint8_t)brk[j];
-            report->iterations[j] = it[j];
-            report->true_residual[j] = res[j];
-            report->relative_residual[j] = rel[j];
+            report->converged[j] = (uint8_t)h.conv[j];
+            report->breakdown[j] = (uint8_t)h.brk[j];
+            report->iterations[j] = h.iters[j];
+            report->true_residual[j] = h.residual[j];
+            report->relative_residual[j] = h.relative[j];
         }
     }
-    if (flags[2]) return fail(KMSD_EINVAL, "metric RHS must be finite");
+    if (h.flags[2]) return fail(KMSD_EINVAL, "metric RHS must be finite");
     if (hst[0]) {
         // Reproduce the reference's message precedence (native.cpp:447-450).
-        std::vector<int> fino(ncols);
-        KMSD_CUDA(cudaMemcpy(fino.data(), c.fino, ncols * sizeof(int), cudaMemcpyDeviceToHost));
         bool representable = true;
-        for (int64_t j = 0; j < ncols; ++j) representable = representable && fino[j];
+        for (int64_t j = 0; j < ncols; ++j) representable = representable && h.fino[j];
         if (!representable)
             return fail(KMSD_EMETRIC,
                         "S solve solution is nonfinite or not representable in complex128 after rescaling");
-        if (flags[3]) return fail(KMSD_EMETRIC, "PCG non-positive/complex curvature breakdown");
+        if (h.flags[3]) return fail(KMSD_EMETRIC, "PCG non-positive/complex curvature breakdown");
         return fail(KMSD_EMETRIC, "S solve failed true-residual acceptance");
     }
     return KMSD_OK;
@@ -1478,6 +1442,9 @@ int kmsd_metric_s::prepare_dev(int64_t b) {
     const int sf = bsr ? (S->bsr64().im ? S_BSR_CPLX : S_BSR_REAL) : S_CSR;
     PcgFn fn = pick(mu_for(mp), nblocks ? maxb : 1, sf, seg, store32 != 0);
     if (!fn) return fail(KMSD_EINVAL, "unsupported metric block size / column count");
+    ResidentPlan plan;
+    if (int rc = resident_plan(this, b, &plan)) return rc;
+    if (plan.form) return KMSD_OK;
     if (!loop_stream) KMSD_CUDA(cudaStreamCreateWithFlags(&loop_stream, cudaStreamNonBlocking));
     if (!check_stream) KMSD_CUDA(cudaStreamCreateWithFlags(&check_stream, cudaStreamNonBlocking));
     return fn(this, nullptr, nullptr, b, 0., 0., 1, nullptr, nullptr, nullptr, nullptr, kPrepare);
@@ -1497,6 +1464,14 @@ int kmsd_metric_s::solve_dev(const double2 *B, double2 *Y, int64_t b, double rto
     const int sf = bsr ? (S->bsr64().im ? S_BSR_CPLX : S_BSR_REAL) : S_CSR;
     PcgFn fn = pick(mu_for(mp), nblocks ? maxb : 1, sf, seg, store32 != 0);
     if (!fn) return fail(KMSD_EINVAL, "unsupported metric block size / column count");
+    ResidentPlan plan;
+    if (int rc = resident_plan(this, b, &plan)) return rc;
+    if (plan.form) {
+        const int rc = resident_solve(this, plan, B, Y, b, rtol, atol, maxiter, s, status,
+                                      static_cast<FailReportFull *>(fail_report));
+        if (!rc) ++calls;
+        return rc;
+    }
     if (!loop_stream) KMSD_CUDA(cudaStreamCreateWithFlags(&loop_stream, cudaStreamNonBlocking));
     if (!check_stream) KMSD_CUDA(cudaStreamCreateWithFlags(&check_stream, cudaStreamNonBlocking));
     FailReportFull *fr = static_cast<FailReportFull *>(fail_report);
@@ -1729,11 +1704,13 @@ void kmsd_metric_destroy(kmsd_metric m) {
     cudaFree(m->bstart);
     cudaFree(m->foff);
     cudaFree(m->factors);
-    for (DevBuf *d : {&m->q, &m->y, &m->r, &m->z, &m->p, &m->sp, &m->t, &m->cols, &m->dcount}) d->release();
+    for (DevBuf *d : {&m->q, &m->y, &m->r, &m->z, &m->p, &m->sp, &m->t, &m->cols, &m->dcount, &m->resident})
+        d->release();
     m->red.partial.release();
     m->red.ticket.release();
     if (m->host_pinned.p) cudaFreeHost(m->host_pinned.p);
     for (auto &kv : m->seg_plans) kv.second.mem.release();
+    for (auto &kv : m->halos) kv.second.mem.release();
     for (auto &kv : m->graphs) cudaGraphExecDestroy(kv.second.first);
     if (m->loop_stream) cudaStreamDestroy(m->loop_stream);
     if (m->check_stream) cudaStreamDestroy(m->check_stream);

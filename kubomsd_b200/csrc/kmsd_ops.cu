@@ -59,7 +59,7 @@ int finish(E *e, cudaStream_t s) {
         }
     }
     if (st[2] != 0) return fail(KMSD_ERUNTIME, "nonfinite Chebyshev propagation; check bounds and solves");
-    if (st[3] != 0) return fail(KMSD_ERUNTIME, "a bounded device wait of the tiled Chebyshev step ran out");
+    if (st[3] != 0) return fail(KMSD_ERUNTIME, "a bounded device wait ran out");
     return KMSD_OK;
 }
 
