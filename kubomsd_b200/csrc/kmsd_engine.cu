@@ -393,6 +393,7 @@ int kmsd_csr_create(int64_t n, const int64_t *indptr, const int64_t *indices, co
     // index/value bytes (lattice Hamiltonians: every row has the same length).
     int64_t lmax = 0;
     for (int64_t r = 0; r < n; ++r) lmax = std::max<int64_t>(lmax, indptr[r + 1] - indptr[r]);
+    A->row_max = (int)lmax;
     const int64_t w = std::max<int64_t>(4, (lmax + 3) / 4 * 4);
     if (!rc && lmax > 0 && w <= 32 && n * w <= nnz + nnz / 4 + 4) {
         const int64_t m = n * w;

@@ -64,6 +64,7 @@ size_t reduce_smem(const RowMap &mp, int C);
 // ------------------------------------------------------------------ CSR
 struct kmsd_csr_s {
     int64_t n = 0, nnz = 0;
+    int row_max = 0;  // entries of the longest row
     int *ptr = nullptr, *idx = nullptr;
     double *re64 = nullptr, *im64 = nullptr;
     float *re32 = nullptr, *im32 = nullptr;  // created on first mixed use
@@ -228,6 +229,7 @@ struct kmsd_engine_s {
     int64_t h_calls = 0, v_calls = 0;
     bool identity = false;
     kmsd::DevBuf ta, tb, bra, hx, t1, t2, t3, t4, t5, psi, vc, inj[3], outw;
+    kmsd::DevBuf cluster;  // column sums of the one-launch moments (kmsd_cluster.cu)
     kmsd::DevBuf ring, corr_partial;  // left-chain ring and partial sums of the correlation tables
     // per axis, the inline velocity's values aligned with H's ELL columns
     // (complex, FP64 and FP32 copies); built on first use, -1: cannot align

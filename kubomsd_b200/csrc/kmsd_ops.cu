@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "kmsd.h"
+#include "kmsd_cluster.cuh"
 #include "kmsd_impl.h"
 #include "kmsd_kernels.cuh"
 #include "kmsd_tile.cuh"
@@ -325,6 +326,27 @@ __global__ void lanczos_scale_kernel(const double2 *w, double2 *v, int64_t n, co
 }
 
 // ---------------------------------------------------------------- moments
+// Moments of a small real operator on an orthogonal basis as one launch
+// (kmsd_cluster.cu); *done says whether that path took the call.
+template <class T>
+int moments_small(E *e, const double2 *B, double *mu, int64_t b, int64_t len, double center, double half, bool doubling,
+                  cudaStream_t s, bool *done) {
+    *done = false;
+    if (!e->identity || e->H->complex_values || len < 2) return KMSD_OK;
+    ClusterPlan pl;
+    int rc = cluster_plan<T>(e->H->n, e->H->row_max, b, doubling, 1, &pl);
+    if (rc || !pl.size) return rc;
+    if (e->cluster.ensure(cluster_scratch(pl, 1, len, doubling))) return KMSD_ECUDA;
+    if (std::is_same<T, float>::value && e->H->ensure_f32()) return KMSD_ECUDA;
+    const ClusterSystem one{0, e->H->n, center, half, mu};
+    rc = cluster_moments<T>(pl, view_of<T>(e->H), e->H->row_max, B, b, len, doubling, nullptr, 1, one,
+                            e->cluster.as<double>(), s);
+    if (rc) return rc;
+    e->h_calls += doubling ? (len + 1) / 2 : len - 1;
+    *done = true;
+    return KMSD_OK;
+}
+
 int moments_impl(E *e, const double2 *B, double *mu, int64_t b, int64_t len, double center, double half, int flags,
                  cudaStream_t s) {
     const int64_t n = e->H->n;
@@ -334,6 +356,11 @@ int moments_impl(E *e, const double2 *B, double *mu, int64_t b, int64_t len, dou
         return fail(KMSD_EINVAL, "moment doubling requires an identity metric (orthogonal basis)");
     double2 *dots = e->dots.as<double2>();
     int rc;
+    bool done = false;
+    if ((rc = e->precision == KMSD_FP64 ? moments_small<double>(e, B, mu, b, len, center, half, doubling, s, &done)
+                                        : moments_small<float>(e, B, mu, b, len, center, half, doubling, s, &done)))
+        return rc;
+    if (done) return KMSD_OK;
     if (e->precision == KMSD_FP64) {
         const double2 *bra = B;
         if (e->identity) {
@@ -871,7 +898,9 @@ int kmsd_engine_create(kmsd_csr h, kmsd_metric m, const int *vel_kind, const kms
 void kmsd_engine_destroy(kmsd_engine e) {
     if (!e) return;
     for (DevBuf *d : {&e->ta, &e->tb, &e->bra, &e->hx, &e->t1, &e->t2, &e->t3, &e->t4, &e->t5, &e->psi, &e->vc,
-                      &e->inj[0], &e->inj[1], &e->inj[2], &e->outw, &e->status, &e->report, &e->dots})
+                      &e->inj[0], &e->inj[1], &e->inj[2], &e->outw, &e->status, &e->report, &e->dots, &e->cluster,
+                      &e->ring, &e->corr_partial, &e->vell64[0], &e->vell64[1], &e->vell64[2], &e->vell32[0],
+                      &e->vell32[1], &e->vell32[2]})
         d->release();
     e->red.partial.release();
     e->red.ticket.release();

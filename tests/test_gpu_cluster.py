@@ -1,0 +1,73 @@
+"""Moments of small operators in one launch (kmsd_cluster.cu) against the oracle,
+at the edges of its row shares, row widths, column groups and sum histories.
+
+Tolerances are the path's own: 1e-10 of the largest moment in FP64, 5e-5 in the
+mixed form (complex64 vectors)."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+from tests.helpers import assert_rel
+
+pytestmark = pytest.mark.gpu
+
+
+def ring(n, reach, seed):
+    """A Hermitian real operator with up to 2 reach + 1 entries per row: rows are
+    short at random, so that padding is used."""
+    rng = np.random.default_rng(seed)
+    A = sp.diags([rng.uniform(-.5, .5, n)], [0]).tolil() if n < 40 else sp.diags([rng.uniform(-.5, .5, n)], [0])
+    A = A.tocsr()
+    for d in range(1, reach + 1):
+        i = np.arange(n)
+        j = (i + d * d * 7) % n
+        keep = (rng.random(n) < .9) & (i != j)
+        B = sp.coo_matrix((np.full(keep.sum(), -1. / d), (i[keep], j[keep])), shape=(n, n)).tocsr()
+        A = A + B + B.T
+    A = A.tocsr()
+    A.sum_duplicates()
+    return A
+
+
+# rows, reach (width 3, 5, 7), columns, moments
+CASES = [(1, 1, 1, 3), (5, 1, 2, 2), (33, 1, 3, 64), (480, 2, 1, 65), (481, 2, 4, 66), (1000, 3, 5, 129), (4096, 2, 8, 130),
+         (9729, 1, 6, 33), (15361, 3, 2, 20), (15360, 3, 33, 9), (20011, 2, 9, 12), (30720, 2, 3, 9), (38912, 1, 2, 9)]
+
+
+@pytest.mark.parametrize("n,reach,b,M", CASES)
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("doubling", [False, True])
+def test_cluster_moments(cuda, n, reach, b, M, precision, doubling):
+    from oracle import kpm_oracle as O
+    from tests.gpu_util import engine
+    H = ring(n, reach, n + b)
+    S = sp.identity(n, format="csr")
+    _, eng, _ = engine(H, S, precision=precision)
+    half = 1.05 * float(abs(H).sum(axis=1).max()) + .1
+    B = np.exp(2j * np.pi * np.random.default_rng(b).random((n, b)))
+    lib = eng.lib
+    before = lib.kmsd_kernel_launches()
+    got = eng.moments(B, M, .05, half, doubling=doubling)
+    launches = lib.kmsd_kernel_launches() - before
+    limit = 16 * (480 if precision == "fp64" else 608) * (4 if H.indptr.size and np.diff(H.indptr).max() < 6 else 2)
+    if n <= limit:
+        assert launches == 1
+    want = O.engine_from_model(H, S).moments(B, M, .05, half)
+    assert_rel(got, want, 1e-10 if precision == "fp64" else 5e-5, f"{n} {b} {M}")
+    np.testing.assert_array_equal(got, eng.moments(B, M, .05, half, doubling=doubling))
+    assert eng.core.h_calls == 2 * ((M + 1) // 2 if doubling else M - 1)
+
+
+def test_complex_and_wide_rows_keep_the_launch_per_step(cuda):
+    from oracle import kpm_oracle as O
+    from tests.gpu_util import engine
+    n = 500
+    S = sp.identity(n, format="csr")
+    B = np.exp(2j * np.pi * np.random.default_rng(1).random((n, 3)))
+    H = ring(n, 2, 1).astype(complex)
+    H = H + 1j * (sp.triu(ring(n, 1, 2), 1) - sp.tril(ring(n, 1, 2), -1))
+    for A in (H.tocsr(), ring(n, 6, 3)):
+        _, eng, _ = engine(A, S)
+        half = 1.05 * float(abs(A).sum(axis=1).max())
+        want = O.engine_from_model(A, S).moments(B, 40, 0., half)
+        assert_rel(eng.moments(B, 40, 0., half), want, 1e-10)
