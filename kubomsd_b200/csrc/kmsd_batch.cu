@@ -10,15 +10,21 @@
 // all steps of a call is captured once into a CUDA graph and replayed on later
 // calls with the same buffers and shape.  `kmsd_batch_tune` times candidate
 // tile sizes and keeps the fastest.
+//
+// Batches whose instances all fit a thread-block cluster take all steps in one
+// launch instead (kmsd_cluster.cu), with no graph and no tiles.
 #include <algorithm>
 #include <cmath>
 #include <chrono>
 #include <cstring>
 #include <map>
 #include <tuple>
+#include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "kmsd.h"
+#include "kmsd_cluster.cuh"
 #include "kmsd_impl.h"
 #include "kmsd_kernels.cuh"
 
@@ -219,6 +225,16 @@ struct kmsd_batch_s {
     double rtol = 1e-10, atol = 0.;
     int maxiter = 1000;
     DevBuf hx, t1, status, report;
+    // One-launch moments (kmsd_cluster.cu) per column count and method, and the
+    // systems of the last call as the device has them.
+    struct Clusters {
+        ClusterPlan plan;
+        DevBuf jobs;
+    };
+    int width = 0;  // entries of the longest row, 0: an instance has complex entries
+    std::map<std::pair<int64_t, bool>, Clusters> clusters;
+    std::vector<ClusterSystem> last_systems;
+    DevBuf systems, sums;
     int64_t general_kernels = 0;  // host-side kernels recorded in the nonorthogonal graph
 };
 
@@ -442,9 +458,52 @@ int general_status(kmsd_batch_s *bt, cudaStream_t s) {
     return KMSD_OK;
 }
 
+// The moments of all instances in one launch, where every instance is small
+// enough for a cluster; *done says whether that path took the call.
+template <class T>
+int run_clusters(kmsd_batch_s *bt, const double2 *B, double *mu, int64_t b, int64_t length, bool doubling, cudaStream_t s,
+                 bool *done) {
+    *done = false;
+    if (bt->width == 0 || length < 2) return KMSD_OK;
+    auto &cl = bt->clusters[{b, doubling}];
+    if (!cl.jobs.p && cl.plan.groups == 0) {
+        std::vector<int64_t> rows(bt->ninst);
+        for (int64_t i = 0; i < bt->ninst; ++i) rows[i] = bt->row_off[i + 1] - bt->row_off[i];
+        std::vector<ClusterJob> jobs;
+        if (int rc = cluster_batch_plan<T>(rows, bt->width, b, doubling, &cl.plan, &jobs)) return rc;
+        if (cl.plan.size == 0) cl.plan.groups = -1;  // decided: does not apply
+        else {
+            if (cl.jobs.ensure(jobs.size() * sizeof(ClusterJob))) return KMSD_ECUDA;
+            KMSD_CUDA(cudaMemcpy(cl.jobs.p, jobs.data(), jobs.size() * sizeof(ClusterJob), cudaMemcpyHostToDevice));
+        }
+    }
+    if (cl.plan.size == 0) return KMSD_OK;
+    std::vector<ClusterSystem> sys(bt->ninst);
+    for (int64_t i = 0; i < bt->ninst; ++i)
+        sys[i] = ClusterSystem{bt->row_off[i], bt->row_off[i + 1] - bt->row_off[i], bt->last_center[i], bt->last_half[i],
+                               mu + (size_t)i * length * b};
+    if (bt->systems.ensure(sys.size() * sizeof(ClusterSystem)) || bt->sums.ensure(cluster_scratch(cl.plan, length, doubling)))
+        return KMSD_ECUDA;
+    if (bt->last_systems.size() != sys.size() ||
+        std::memcmp(bt->last_systems.data(), sys.data(), sys.size() * sizeof(ClusterSystem)) != 0) {
+        KMSD_CUDA(cudaMemcpyAsync(bt->systems.p, sys.data(), sys.size() * sizeof(ClusterSystem), cudaMemcpyHostToDevice, s));
+        bt->last_systems.swap(sys);
+    }
+    CsrView<T> H;
+    if constexpr (std::is_same<T, float>::value) H = bt->G.view32();
+    else H = bt->G.view64();
+    const int rc = cluster_moments<T>(cl.plan, H, bt->width, B, b, length, doubling, bt->systems.as<ClusterSystem>(),
+                                      cl.jobs.as<ClusterJob>(), ClusterSystem{}, bt->sums.as<double>(), s);
+    *done = rc == KMSD_OK;
+    return rc;
+}
+
 template <class T>
 int run_batch(kmsd_batch_s *bt, const double2 *B, double *mu, int64_t b, int64_t length, bool doubling,
               cudaStream_t s, bool use_graph) {
+    bool done = false;
+    if (int rc = run_clusters<T>(bt, B, mu, b, length, doubling, s, &done)) return rc;
+    if (done) return KMSD_OK;
     constexpr int C = Unit<T>::C;
     const int U = (int)((b + C - 1) / C);
     const RowMap mp = make_map(U, kThreads);
@@ -624,8 +683,10 @@ int kmsd_batch_create(int64_t ninst, const kmsd_csr *H, int precision, int64_t t
         bt->row_off[i + 1] = bt->row_off[i] + H[i]->n;
         bt->nnz_off[i + 1] = bt->nnz_off[i] + H[i]->nnz;
         cplx = cplx || H[i]->complex_values;
+        bt->width = std::max(bt->width, H[i]->row_max);
         if (H[i]->ell_w != w) w = 0;
     }
+    if (cplx) bt->width = 0;
     bt->n = bt->row_off[ninst];
     bt->nnz = bt->nnz_off[ninst];
     if (bt->n >= INT32_MAX || bt->nnz >= INT32_MAX) {
@@ -718,8 +779,9 @@ void kmsd_batch_destroy(kmsd_batch bt) {
         cudaFree(p);
     G = kmsd_csr_s();
     for (DevBuf *d : {&bt->dcenter, &bt->dhalf, &bt->ta, &bt->tb, &bt->bra, &bt->partial, &bt->tilemem, &bt->hx,
-                      &bt->t1, &bt->status, &bt->report})
+                      &bt->t1, &bt->status, &bt->report, &bt->systems, &bt->sums})
         d->release();
+    for (auto &kv : bt->clusters) kv.second.jobs.release();
     delete bt;
 }
 

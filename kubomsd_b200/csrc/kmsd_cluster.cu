@@ -7,7 +7,8 @@
 // out the rows, T_k and T_{k-1} stay in their shared memory, a thread keeps the
 // entries of its rows (column addresses and values) in registers, neighbours on
 // another CTA are read through distributed shared memory, and the CTAs meet at
-// the cluster's hardware barrier once per step (about 0.2 us).  The column sums
+// the cluster's hardware barrier once per step (about 0.2 us).  Small systems
+// share out the columns over the warps too.  The column sums
 // of a step are reduced in the warp, then by a warp of its own during the next
 // step, and leave shared memory every kHist steps, so that no global store
 // stands before the barrier.
@@ -16,9 +17,10 @@
 // fused multiply-adds, store) and the meeting, 0.8-1 us a step; for many, the
 // shared-memory traffic, (W + 3) elements per row and column.  A cluster of up to
 // 16 CTAs whose threads own up to 4 rows covers about 30,000 rows.  M = 512
-// direct moments of 4,096 sites x 8 complex128 columns took 0.55 ms against 4.33
+// direct moments of 4,096 sites x 8 complex128 columns took 0.52 ms against 4.33
 // with a launch per step; 511 of 16,129 x 31 complex64 by the product identity
-// 0.89 ms against 5.39.  Within its reach it was the faster one everywhere: from
+// 0.81 ms against 5.39; 256 of 24 lattices of 576 to 25,600 sites x 16 complex64
+// in one launch 2.28 ms against 9.10.  Within its reach it was the faster one everywhere: from
 // 512 to 30,720 rows and 1 to 256 columns by 1.5 (28,900 x 256) to 10 times.
 //
 // The arithmetic of an element is that of cheb_step_kernel, entry by entry, so
@@ -26,9 +28,11 @@
 // (fixed) order.
 #include <algorithm>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <utility>
 
 #include "kmsd_cluster.cuh"
 
@@ -49,9 +53,10 @@ template <class T> struct ClusterArgs {
     CsrView<T> H;
     const double2 *B;
     int64_t b;
-    const ClusterSystem *systems;  // nullptr: one
+    const ClusterSystem *systems;  // nullptr: `one`, its columns in groups of `cols`
+    const ClusterJob *jobs;        // per cluster, with `systems`
     ClusterSystem one;
-    int groups, cols, rows;
+    int cols;  // most columns of a cluster
     int64_t length;
     int steps;
     double *partial;  // [cluster][step][CTA][2 * cols]
@@ -70,13 +75,15 @@ __device__ __forceinline__ unsigned remote_address(unsigned at, unsigned rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(at), "r"(rank));
     return r;
 }
-// An element from any CTA's shared memory.
-__device__ __forceinline__ double2 load_far(unsigned at, double2) {
+// An element from any CTA's shared memory, this one's too: addresses of the own
+// CTA take the same load at the same speed, so no read needs a branch (one branch
+// per row made 4,096 x 8 4 % and 16,129 x 31 7 % slower).
+__device__ __forceinline__ double2 load_any(unsigned at, double2) {
     double2 v;
     asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(at));
     return v;
 }
-__device__ __forceinline__ float2 load_far(unsigned at, float2) {
+__device__ __forceinline__ float2 load_any(unsigned at, float2) {
     float2 v;
     asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(at));
     return v;
@@ -104,6 +111,12 @@ __device__ __forceinline__ bool warp_sums(double (&v)[NV], int lane, int &which)
     return (lane & rest) == 0;
 }
 
+// Sets of warps that share out a cluster's columns (1: all warps own rows).
+__host__ __device__ inline int column_sets(int warps, int rows) {
+    const int wr = rows > 32 ? (rows + 31) / 32 : 1;
+    return 2 * wr <= warps ? warps / wr : 1;
+}
+
 // Rows of up to W entries, RPT rows per thread, CG columns at a time.
 template <class T, bool DIRECT, int W, int RPT, int CG>
 __global__ void __launch_bounds__(kMaxCompute<T> + 32, 1) cluster_moments_kernel(const ClusterArgs<T> a) {
@@ -114,14 +127,26 @@ __global__ void __launch_bounds__(kMaxCompute<T> + 32, 1) cluster_moments_kernel
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
     const int cluster = blockIdx.x / size;
-    const ClusterSystem sys = a.systems ? a.systems[cluster / a.groups] : a.one;
-    const int c0 = (cluster % a.groups) * a.cols;
-    const int cols = min(a.cols, (int)(a.b - c0));
+    ClusterSystem sys = a.one;
+    int c0 = cluster * a.cols, cols = min(a.cols, (int)(a.b - c0));
+    if (a.systems) {
+        const ClusterJob job = a.jobs[cluster];
+        sys = a.systems[job.system];
+        c0 = job.c0;
+        cols = job.cols;
+    }
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int compute = blockDim.x - 32, warps = compute / 32;
-    const int rows = a.rows;
+    const int compute = blockDim.x - 32;
+    const int rows = (int)((sys.n + size - 1) / size);
     const int mine = max(0, min(rows, (int)(sys.n - (int64_t)rank * rows)));
-    const unsigned plane = (unsigned)rows * sizeof(V), block = plane * a.cols;
+    // Where the rows take at most half of the warps, sets of warps share out the
+    // columns: warp w is warp `own` of set w / wr.
+    const int cwarps = compute / 32, wr = max(1, (rows + 31) / 32), sets = column_sets(cwarps, rows);
+    const int set = sets > 1 ? warp / wr : 0, own = sets > 1 ? warp - set * wr : warp;
+    const int at_row = own * 32 + lane;  // this thread's first row; the next ones follow `compute` apart
+    const int warps = min(cwarps, (mine + 31) / 32);  // of a set that own rows
+    const bool works = warp < cwarps && set < sets && own < warps && set * CG < cols;
+    const unsigned plane = (unsigned)rows * sizeof(V), block = plane * cols;
     const unsigned base = (unsigned)__cvta_generic_to_shared(sm);
     // [T_k | T_{k-1} (| bra)][column][row], the sums of the warps (two steps), the history
     V *vec = reinterpret_cast<V *>(sm);
@@ -134,14 +159,12 @@ __global__ void __launch_bounds__(kMaxCompute<T> + 32, 1) cluster_moments_kernel
     // (short rows read their own element times zero)
     unsigned at[RPT][W];
     T val[RPT][W];
-    bool far[RPT];  // a row of this warp has a column on another CTA
 #pragma unroll
     for (int i = 0; i < RPT; ++i) {
-        const int r = i * compute + tid;
-        const bool on = tid < compute && r < mine;
+        const int r = i * compute + at_row;
+        const bool on = works && r < mine;
         const int64_t g = sys.row0 + (int64_t)rank * rows + r;
         const int k0 = on ? a.H.ptr[g] : 0, k1 = on ? a.H.ptr[g + 1] : 0;
-        bool away = false;
 #pragma unroll
         for (int j = 0; j < W; ++j) {
             at[i][j] = base + (on ? (unsigned)r * (unsigned)sizeof(V) : 0u);
@@ -150,13 +173,9 @@ __global__ void __launch_bounds__(kMaxCompute<T> + 32, 1) cluster_moments_kernel
                 const int rel = (int)(a.H.idx[k0 + j] - sys.row0), owner = rel / rows, loc = rel - owner * rows;
                 val[i][j] = a.H.re[k0 + j];
                 at[i][j] = base + (unsigned)loc * (unsigned)sizeof(V);
-                if (owner != (int)rank) {
-                    at[i][j] = remote_address(at[i][j], owner);
-                    away = true;
-                }
+                if (owner != (int)rank) at[i][j] = remote_address(at[i][j], owner);
             }
         }
-        far[i] = __any_sync(0xffffffffu, away);
     }
     for (int i = tid; i < mine * cols; i += blockDim.x) {
         const int r = i / cols, c = i - r * cols;
@@ -165,9 +184,9 @@ __global__ void __launch_bounds__(kMaxCompute<T> + 32, 1) cluster_moments_kernel
         w.x = (T)v.x;
         w.y = (T)v.y;
         vec[(size_t)c * rows + r] = w;
-        if (DIRECT) vec[(size_t)(2 * a.cols + c) * rows + r] = w;
+        if (DIRECT) vec[(size_t)(2 * cols + c) * rows + r] = w;
         w.x = w.y = T(0);
-        vec[(size_t)(a.cols + c) * rows + r] = w;  // "T_{-1}": the first step is t - 0
+        vec[(size_t)(cols + c) * rows + r] = w;  // "T_{-1}": the first step is t - 0
     }
     cluster_sync_all();
 
@@ -194,19 +213,19 @@ __global__ void __launch_bounds__(kMaxCompute<T> + 32, 1) cluster_moments_kernel
     auto put = [&](double (&s)[NS * CG], int c, int sum) {
         int which;
         if (warp_sums<NS * CG>(s, lane, which) && c + which / NS < cols)
-            red[((sum & 3) * warps + warp) * nv + c * NS + which] = s[0];
+            red[((sum & 3) * warps + own) * nv + c * NS + which] = s[0];
     };
     // DIRECT: sum 0 is <B, B>, sum k is <B, T_k>; else sum k - 1 holds <T_{k-1}, T_{k-1}> and <T_{k-1}, T_k>
     int sums = 0;
     if (DIRECT) {
-        if (tid < compute)
-            for (int c = 0; c < cols; c += CG) {
+        if (works)
+            for (int c = set * CG; c < cols; c += sets * CG) {
                 double s[NS * CG];
 #pragma unroll
                 for (int q = 0; q < NS * CG; ++q) {
                     s[q] = 0.;
                     if (c + q < cols)
-                        for (int r = tid; r < mine; r += compute) {
+                        for (int r = at_row; r < mine; r += compute) {
                             const V x = vec[(size_t)(c + q) * rows + r];
                             s[q] += (double)x.x * (double)x.x + (double)x.y * (double)x.y;
                         }
@@ -219,9 +238,9 @@ __global__ void __launch_bounds__(kMaxCompute<T> + 32, 1) cluster_moments_kernel
     unsigned cur = 0;  // offset of T_{k-1}; T_k goes to the other block, over T_{k-2}
     T two = T(1);      // 2, and 1 in the first step
     for (int k = 1; k <= a.steps; ++k) {
-        if (tid < compute) {
+        if (works) {
             const unsigned nxt = block - cur;
-            for (int c = 0; c < cols; c += CG) {
+            for (int c = set * CG; c < cols; c += sets * CG) {
                 double s[NS * CG];
 #pragma unroll
                 for (int q = 0; q < NS * CG; ++q) s[q] = 0.;
@@ -231,18 +250,12 @@ __global__ void __launch_bounds__(kMaxCompute<T> + 32, 1) cluster_moments_kernel
                         const unsigned off = (unsigned)(c + q) * plane, from = off + cur;
 #pragma unroll
                         for (int i = 0; i < RPT; ++i) {
-                            const int r = i * compute + tid;
+                            const int r = i * compute + at_row;
                             if (RPT == 1 || i == 0 || r < mine) {  // (idle lanes of the first row repeat row 0's reads)
                                 const unsigned me = off + (unsigned)(r < mine ? r : 0) * (unsigned)sizeof(V);
                                 V xv[W];
-                                if (far[i]) {
 #pragma unroll
-                                    for (int j = 0; j < W; ++j) xv[j] = load_far(at[i][j] + from, V{});
-                                } else {
-#pragma unroll
-                                    for (int j = 0; j < W; ++j)
-                                        xv[j] = *reinterpret_cast<const V *>(sm + (at[i][j] + from - base));
-                                }
+                                for (int j = 0; j < W; ++j) xv[j] = load_any(at[i][j] + from, V{});
                                 const V x = *reinterpret_cast<const V *>(sm + me + cur);
                                 V *dst = reinterpret_cast<V *>(sm + me + nxt);
                                 const V pv = *dst;  // T_{k-2}
@@ -270,12 +283,12 @@ __global__ void __launch_bounds__(kMaxCompute<T> + 32, 1) cluster_moments_kernel
                         }
                     }
                 }
-                if (c + CG >= cols) cluster_arrive();  // T_k is written: its sums overlap the meeting
+                if (c + sets * CG >= cols) cluster_arrive();  // T_k is written: its sums overlap the meeting
                 put(s, c, sums);
             }
         } else {
             cluster_arrive();
-            if (sums > 1) collect(sums - 2, false);  // written before the last meeting
+            if (tid >= compute && sums > 1) collect(sums - 2, false);  // written before the last meeting
         }
         cluster_wait();
         ++sums;
@@ -323,9 +336,13 @@ const void *pick_shape(int rpt, int cg) {
             return cg == 1 ? (const void *)cluster_moments_kernel<T, DIRECT, W, 2, 1>
                            : (const void *)cluster_moments_kernel<T, DIRECT, W, 2, 4>;
     }
-    if constexpr (W < kClusterWidth)
+    if constexpr (W < kClusterWidth) {
+        if (rpt == 3)
+            return cg == 1 ? (const void *)cluster_moments_kernel<T, DIRECT, W, 3, 1>
+                           : (const void *)cluster_moments_kernel<T, DIRECT, W, 3, 4>;
         return cg == 1 ? (const void *)cluster_moments_kernel<T, DIRECT, W, 4, 1>
                        : (const void *)cluster_moments_kernel<T, DIRECT, W, 4, 4>;
+    }
     return nullptr;
 }
 // Rows a thread may own: the entries of four rows of eight do not fit its registers.
@@ -383,17 +400,38 @@ int active_clusters(const void *kernel, int size, int threads, size_t smem) {
     return n;
 }
 
+template <class T> int rows_per_thread(int64_t rows) { return (int)((rows + kMaxCompute<T> - 1) / kMaxCompute<T>); }
+int cluster_threads(int64_t rows, int rpt) { return (int)(((rows + rpt - 1) / rpt + 31) / 32 * 32) + 32; }
+// Shared memory of the vector blocks, and of the sums of a CTA.
+template <class T> size_t vec_bytes(int64_t rows, int cols, bool doubling) {
+    return ((size_t)rows * cols * 2 * sizeof(T) * (doubling ? 2 : 3) + 15) / 16 * 16;
+}
+size_t sum_bytes(int threads, int cols, bool doubling) {
+    return (size_t)(4 * (threads / 32 - 1) + kHist) * (doubling ? 2 : 1) * cols * sizeof(double);
+}
+// Cycles of a step of a cluster whose CTAs have `threads`: the meeting, then for
+// each (row, column) of a thread the chain of its loads and arithmetic, or the
+// shared-memory traffic of all warps where that is more (fitted to 0.9 us for
+// 256 rows x 1 complex128 column of a CTA and 2.8 us for 1009 x 5 complex64).
+template <class T> double step_cycles(int64_t rows, int cols, int width, bool doubling, int size, int threads) {
+    const int warps = threads / 32 - 1, sets = column_sets(warps, (int)rows);
+    const int64_t items = (cols + sets - 1) / sets * ((rows + 32 * warps - 1) / (32 * warps));
+    const int busy = std::min<int64_t>(warps, sets * ((rows + 31) / 32));
+    const double traffic = busy * (width + (doubling ? 3. : 4.)) * (2 * sizeof(T)) * 32 / 128.;
+    return (size > 1 ? 1000. : 600.) + items * std::max(400., traffic);
+}
+
 }  // namespace
 
 namespace kmsd {
 
 template <class T>
-int cluster_plan(int64_t n, int width, int64_t b, bool doubling, int64_t systems, ClusterPlan *out) {
+int cluster_plan(int64_t n, int width, int64_t b, bool doubling, ClusterPlan *out) {
     *out = ClusterPlan{};
     if (width < 1 || width > kClusterWidth) return KMSD_OK;
     static std::mutex lock;
-    static std::map<std::tuple<int64_t, int, int64_t, bool, int64_t>, ClusterPlan> cache;
-    const auto key = std::make_tuple(n, width, b, doubling, systems);
+    static std::map<std::tuple<int64_t, int, int64_t, bool>, ClusterPlan> cache;
+    const auto key = std::make_tuple(n, width, b, doubling);
     {
         std::lock_guard<std::mutex> guard(lock);
         const auto it = cache.find(key);
@@ -402,30 +440,22 @@ int cluster_plan(int64_t n, int width, int64_t b, bool doubling, int64_t systems
             return KMSD_OK;
         }
     }
-    const int elem = 2 * sizeof(T), blocks = doubling ? 2 : 3, ns = doubling ? 2 : 1;
     double best = 0.;
     for (int size : {16, 8, 4, 2, 1}) {
         const int64_t rows = (n + size - 1) / size;
         if (rows > most_rows(width) * kMaxCompute<T>) continue;
-        const int rpt = rows <= kMaxCompute<T> ? 1 : rows <= 2 * kMaxCompute<T> ? 2 : 4;
-        const int compute = (int)(((rows + rpt - 1) / rpt + 31) / 32 * 32), threads = compute + 32;
+        const int rpt = rows_per_thread<T>(rows), threads = cluster_threads(rows, rpt);
         for (int cols = 1; cols <= std::min<int64_t>(b, 32); ++cols) {
             const int cg = cols == 1 ? 1 : 4;
-            const size_t vec = ((size_t)rows * cols * elem * blocks + 15) / 16 * 16;
-            const size_t smem = vec + (size_t)(4 * (compute / 32) + kHist) * ns * cols * 8;
+            const size_t smem = vec_bytes<T>(rows, cols, doubling) + sum_bytes(threads, cols, doubling);
             if (smem > smem_limit()) break;
             const int64_t groups = (b + cols - 1) / cols;
             const int act = active_clusters(pick_kernel<T>(!doubling, width, rpt, cg), size, threads, smem);
             if (act < 1) continue;
-            const int64_t waves = (groups * systems + act - 1) / act;
-            // cycles of a step: the chain of one row and the meeting, then the
-            // shared-memory traffic (fitted to 0.8 us for 64 rows x 1 column of a
-            // CTA and 3.1 us for 1009 x 5 complex64)
-            const double step = (size > 1 ? 1300. : 900.) + (double)rows * cols * (width + (doubling ? 3 : 4)) * elem / 75.;
-            const double cost = step * waves;
+            const double cost = step_cycles<T>(rows, cols, width, doubling, size, threads) * ((groups + act - 1) / act);
             if (out->size == 0 || cost < best) {
                 best = cost;
-                *out = ClusterPlan{size, (int)rows, cols, (int)groups, rpt, threads, cg, smem};
+                *out = ClusterPlan{size, cols, (int)groups, rpt, threads, cg, smem};
             }
         }
     }
@@ -435,31 +465,91 @@ int cluster_plan(int64_t n, int width, int64_t b, bool doubling, int64_t systems
     return KMSD_OK;
 }
 
-size_t cluster_scratch(const ClusterPlan &pl, int64_t systems, int64_t length, bool doubling) {
+// Systems of several sizes in one launch: a cluster takes as many columns of a
+// system as keep its step below a common length, the longest jobs first.  The
+// cluster size and that length are the ones with the shortest schedule on the
+// clusters that run at once.
+template <class T>
+int cluster_batch_plan(const std::vector<int64_t> &rows_of, int width, int64_t b, bool doubling, ClusterPlan *out,
+                       std::vector<ClusterJob> *jobs) {
+    *out = ClusterPlan{};
+    if (width < 1 || width > kClusterWidth) return KMSD_OK;
+    const int64_t biggest = *std::max_element(rows_of.begin(), rows_of.end());
+    double best = 0.;
+    for (int size : {16, 8, 4, 2, 1}) {
+        const int64_t rows = (biggest + size - 1) / size;
+        if (rows > most_rows(width) * kMaxCompute<T>) continue;
+        const int rpt = rows_per_thread<T>(rows), threads = cluster_threads(rows, rpt);
+        double last = 0.;
+        for (int most = 1; most <= std::min<int64_t>(b, 32); ++most) {
+            const double length = step_cycles<T>(rows, most, width, doubling, size, threads);
+            // columns of each system, and what they need
+            std::vector<std::pair<double, ClusterJob>> list;
+            size_t vec = 0;
+            int cols = 0;
+            for (size_t i = 0; i < rows_of.size(); ++i) {
+                const int64_t r = (rows_of[i] + size - 1) / size;
+                int c = 1;
+                while (c < std::min<int64_t>(b, 32) && step_cycles<T>(r, c + 1, width, doubling, size, threads) <= length) ++c;
+                const int groups = (int)((b + c - 1) / c);
+                c = (int)((b + groups - 1) / groups);
+                cols = std::max(cols, c);
+                vec = std::max(vec, vec_bytes<T>(r, c, doubling));
+                for (int c0 = 0; c0 < b; c0 += c)
+                    list.push_back({step_cycles<T>(r, std::min<int>(c, (int)b - c0), width, doubling, size, threads),
+                                    ClusterJob{(int)i, c0, std::min<int>(c, (int)b - c0), 0}});
+            }
+            const size_t smem = vec + sum_bytes(threads, cols, doubling);
+            if (smem > smem_limit()) break;
+            const int cg = cols == 1 ? 1 : 4;
+            const int act = active_clusters(pick_kernel<T>(!doubling, width, rpt, cg), size, threads, smem);
+            if (act < 1) continue;
+            std::stable_sort(list.begin(), list.end(), [](const auto &x, const auto &y) { return x.first > y.first; });
+            std::vector<double> busy(act, 0.);  // a heap of the clusters' finishing times
+            double end = 0.;
+            for (const auto &j : list) {
+                std::pop_heap(busy.begin(), busy.end(), std::greater<double>());
+                busy.back() += j.first;
+                end = std::max(end, busy.back());
+                std::push_heap(busy.begin(), busy.end(), std::greater<double>());
+            }
+            if (out->size == 0 || end < best) {
+                best = end;
+                *out = ClusterPlan{size, cols, (int)list.size(), rpt, threads, cg, smem};
+                jobs->clear();
+                for (const auto &j : list) jobs->push_back(j.second);
+            }
+            if (last > 0. && end > 2. * last) break;
+            last = end;
+        }
+    }
+    return KMSD_OK;
+}
+
+size_t cluster_scratch(const ClusterPlan &pl, int64_t length, bool doubling) {
     const int64_t sums = doubling ? (length + 1) / 2 : length;
-    return (size_t)pl.groups * systems * sums * pl.size * (doubling ? 2 : 1) * pl.cols * sizeof(double);
+    return (size_t)pl.groups * sums * pl.size * (doubling ? 2 : 1) * pl.cols * sizeof(double);
 }
 
 template <class T>
 int cluster_moments(const ClusterPlan &pl, const CsrView<T> &H, int width, const double2 *B, int64_t b, int64_t length,
-                    bool doubling, const ClusterSystem *systems, int64_t count, const ClusterSystem &one, double *scratch,
-                    cudaStream_t s) {
+                    bool doubling, const ClusterSystem *systems, const ClusterJob *jobs, const ClusterSystem &one,
+                    double *scratch, cudaStream_t s) {
     ClusterArgs<T> a;
     std::memset(&a, 0, sizeof(a));
     a.H = H;
     a.B = B;
     a.b = b;
     a.systems = systems;
+    a.jobs = jobs;
     a.one = one;
-    a.groups = pl.groups;
     a.cols = pl.cols;
-    a.rows = pl.rows;
     a.length = length;
     a.steps = (int)(doubling ? (length + 1) / 2 : length - 1);
     a.partial = scratch;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
-    cluster_config(cfg, at, (int)(pl.groups * count) * pl.size, pl.size, pl.threads, pl.smem);
+    cluster_config(cfg, at, pl.groups * pl.size, pl.size, pl.threads, pl.smem);
     cfg.stream = s;
     void *args[] = {&a};
     KMSD_CUDA(cudaLaunchKernelExC(&cfg, pick_kernel<T>(!doubling, width, pl.rpt, pl.cg), args));
@@ -467,11 +557,15 @@ int cluster_moments(const ClusterPlan &pl, const CsrView<T> &H, int width, const
     return KMSD_OK;
 }
 
-template int cluster_plan<double>(int64_t, int, int64_t, bool, int64_t, ClusterPlan *);
-template int cluster_plan<float>(int64_t, int, int64_t, bool, int64_t, ClusterPlan *);
-template int cluster_moments<double>(const ClusterPlan &, const CsrView<double> &, int, const double2 *, int64_t, int64_t, bool,
-                                     const ClusterSystem *, int64_t, const ClusterSystem &, double *, cudaStream_t);
-template int cluster_moments<float>(const ClusterPlan &, const CsrView<float> &, int, const double2 *, int64_t, int64_t, bool,
-                                    const ClusterSystem *, int64_t, const ClusterSystem &, double *, cudaStream_t);
+#define KMSD_CLUSTER_INSTANCES(T)                                                                                       \
+    template int cluster_plan<T>(int64_t, int, int64_t, bool, ClusterPlan *);                                           \
+    template int cluster_batch_plan<T>(const std::vector<int64_t> &, int, int64_t, bool, ClusterPlan *,                 \
+                                       std::vector<ClusterJob> *);                                                      \
+    template int cluster_moments<T>(const ClusterPlan &, const CsrView<T> &, int, const double2 *, int64_t, int64_t,    \
+                                    bool, const ClusterSystem *, const ClusterJob *, const ClusterSystem &, double *,   \
+                                    cudaStream_t);
+KMSD_CLUSTER_INSTANCES(double)
+KMSD_CLUSTER_INSTANCES(float)
+#undef KMSD_CLUSTER_INSTANCES
 
 }  // namespace kmsd

@@ -334,12 +334,12 @@ int moments_small(E *e, const double2 *B, double *mu, int64_t b, int64_t len, do
     *done = false;
     if (!e->identity || e->H->complex_values || len < 2) return KMSD_OK;
     ClusterPlan pl;
-    int rc = cluster_plan<T>(e->H->n, e->H->row_max, b, doubling, 1, &pl);
+    int rc = cluster_plan<T>(e->H->n, e->H->row_max, b, doubling, &pl);
     if (rc || !pl.size) return rc;
-    if (e->cluster.ensure(cluster_scratch(pl, 1, len, doubling))) return KMSD_ECUDA;
+    if (e->cluster.ensure(cluster_scratch(pl, len, doubling))) return KMSD_ECUDA;
     if (std::is_same<T, float>::value && e->H->ensure_f32()) return KMSD_ECUDA;
     const ClusterSystem one{0, e->H->n, center, half, mu};
-    rc = cluster_moments<T>(pl, view_of<T>(e->H), e->H->row_max, B, b, len, doubling, nullptr, 1, one,
+    rc = cluster_moments<T>(pl, view_of<T>(e->H), e->H->row_max, B, b, len, doubling, nullptr, nullptr, one,
                             e->cluster.as<double>(), s);
     if (rc) return rc;
     e->h_calls += doubling ? (len + 1) / 2 : len - 1;

@@ -71,3 +71,25 @@ def test_complex_and_wide_rows_keep_the_launch_per_step(cuda):
         half = 1.05 * float(abs(A).sum(axis=1).max())
         want = O.engine_from_model(A, S).moments(B, 40, 0., half)
         assert_rel(eng.moments(B, 40, 0., half), want, 1e-10)
+
+
+@pytest.mark.parametrize("precision,doubling", [("fp64", False), ("fp64", True), ("mixed", False), ("mixed", True)])
+@pytest.mark.parametrize("sizes,b,M", [((1, 40, 700, 33), 5, 70), ((600, 5000, 20011, 64, 97), 9, 12), ((300,) * 20, 2, 66)])
+def test_cluster_batch(cuda, sizes, b, M, precision, doubling):
+    # every instance with its own window, all in one launch, against separate calls
+    from kubomsd_b200.batch import B200Batch
+    from tests.gpu_util import engine
+    Hs = [ring(n, 2, 50 + i) for i, n in enumerate(sizes)]
+    halves = [1.05 * float(abs(H).sum(axis=1).max()) + .1 for H in Hs]
+    centers = [.01 * i for i in range(len(sizes))]
+    rng = np.random.default_rng(b)
+    Bs = [np.exp(2j * np.pi * rng.random((n, b))) for n in sizes]
+    bt = B200Batch(Hs, precision=precision)
+    before = bt.lib.kmsd_kernel_launches()
+    got = bt.moments(Bs, M, centers, halves, doubling=doubling).cpu().numpy()
+    assert bt.lib.kmsd_kernel_launches() - before == 1
+    for i, H in enumerate(Hs):
+        _, eng, _ = engine(H, sp.identity(sizes[i], format="csr"), precision=precision)
+        want = eng.moments(Bs[i], M, centers[i], halves[i], doubling=doubling)
+        # the same elements, the FP64 sums in another order
+        assert_rel(got[i], want, 1e-13, f"instance {i}")
