@@ -41,14 +41,6 @@ using namespace kmsd;
 namespace {
 
 constexpr int kHist = 64;        // steps whose sums are held in shared memory
-// Threads that own rows (one more warp sums): what 96 (complex64) or 128
-// (complex128) registers a thread allow.
-template <class T> constexpr int kMaxCompute = sizeof(T) == 4 ? 608 : 480;
-
-template <class T> struct Cx;
-template <> struct Cx<double> { using type = double2; };
-template <> struct Cx<float> { using type = float2; };
-
 template <class T> struct ClusterArgs {
     CsrView<T> H;
     const double2 *B;
@@ -61,33 +53,6 @@ template <class T> struct ClusterArgs {
     int steps;
     double *partial;  // [cluster][step][CTA][2 * cols]
 };
-
-// The cluster's meeting in two halves: what lies between them overlaps the
-// meeting and becomes visible with the next one.
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
-__device__ __forceinline__ void cluster_sync_all() {
-    cluster_arrive();
-    cluster_wait();
-}
-__device__ __forceinline__ unsigned remote_address(unsigned at, unsigned rank) {
-    unsigned r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(at), "r"(rank));
-    return r;
-}
-// An element from any CTA's shared memory, this one's too: addresses of the own
-// CTA take the same load at the same speed, so no read needs a branch (one branch
-// per row made 4,096 x 8 4 % and 16,129 x 31 7 % slower).
-__device__ __forceinline__ double2 load_any(unsigned at, double2) {
-    double2 v;
-    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(at));
-    return v;
-}
-__device__ __forceinline__ float2 load_any(unsigned at, float2) {
-    float2 v;
-    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(at));
-    return v;
-}
 
 // Sums NV values over the lanes of a warp; the lane whose low bits are zero
 // returns true and holds the sum of value `which` in v[0].  Halving the values
@@ -109,12 +74,6 @@ __device__ __forceinline__ bool warp_sums(double (&v)[NV], int lane, int &which)
     const int rest = 2 * off - 1;
     for (; off > 0; off /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
     return (lane & rest) == 0;
-}
-
-// Sets of warps that share out a cluster's columns (1: all warps own rows).
-__host__ __device__ inline int column_sets(int warps, int rows) {
-    const int wr = rows > 32 ? (rows + 31) / 32 : 1;
-    return 2 * wr <= warps ? warps / wr : 1;
 }
 
 // Rows of up to W entries, RPT rows per thread, CG columns at a time.
@@ -354,52 +313,6 @@ const void *pick_kernel(bool direct, int width, int rpt, int cg) {
     return direct ? pick_shape<T, true, 8>(rpt, cg) : pick_shape<T, false, 8>(rpt, cg);
 }
 
-// Dynamic shared memory a CTA may have on this device.
-size_t smem_limit() {
-    static const size_t limit = [] {
-        int dev = 0, optin = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-        return (size_t)optin - 1024;
-    }();
-    return limit;
-}
-
-void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, int ctas, int size, int threads, size_t smem) {
-    cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = size;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-}
-
-// Clusters of this shape that run at once (cached; also sets the kernel's
-// attributes on first use).
-int active_clusters(const void *kernel, int size, int threads, size_t smem) {
-    static std::mutex lock;
-    static std::map<std::tuple<const void *, int, int, size_t>, int> cache;
-    std::lock_guard<std::mutex> guard(lock);
-    const auto key = std::make_tuple(kernel, size, threads, smem);
-    auto it = cache.find(key);
-    if (it != cache.end()) return it->second;
-    int n = 0;
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
-    cluster_config(cfg, at, size, size, threads, smem);
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_limit()) != cudaSuccess ||
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        n = 0;
-    }
-    if (cache.size() >= 4096) cache.clear();
-    cache[key] = n;
-    return n;
-}
-
 template <class T> int rows_per_thread(int64_t rows) { return (int)((rows + kMaxCompute<T> - 1) / kMaxCompute<T>); }
 int cluster_threads(int64_t rows, int rpt) { return (int)(((rows + rpt - 1) / rpt + 31) / 32 * 32) + 32; }
 // Shared memory of the vector blocks, and of the sums of a CTA.
@@ -425,6 +338,49 @@ template <class T> double step_cycles(int64_t rows, int cols, int width, bool do
 
 namespace kmsd {
 
+size_t cluster_smem_limit() {
+    static const size_t limit = [] {
+        int dev = 0, optin = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        return (size_t)optin - 1024;
+    }();
+    return limit;
+}
+
+void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, int ctas, int size, int threads, size_t smem) {
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = size;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+}
+
+int active_clusters(const void *kernel, int size, int threads, size_t smem) {
+    static std::mutex lock;
+    static std::map<std::tuple<const void *, int, int, size_t>, int> cache;
+    std::lock_guard<std::mutex> guard(lock);
+    const auto key = std::make_tuple(kernel, size, threads, smem);
+    auto it = cache.find(key);
+    if (it != cache.end()) return it->second;
+    int n = 0;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    cluster_config(cfg, at, size, size, threads, smem);
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cluster_smem_limit()) != cudaSuccess ||
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    if (cache.size() >= 4096) cache.clear();
+    cache[key] = n;
+    return n;
+}
+
 template <class T>
 int cluster_plan(int64_t n, int width, int64_t b, bool doubling, ClusterPlan *out) {
     *out = ClusterPlan{};
@@ -448,7 +404,7 @@ int cluster_plan(int64_t n, int width, int64_t b, bool doubling, ClusterPlan *ou
         for (int cols = 1; cols <= std::min<int64_t>(b, 32); ++cols) {
             const int cg = cols == 1 ? 1 : 4;
             const size_t smem = vec_bytes<T>(rows, cols, doubling) + sum_bytes(threads, cols, doubling);
-            if (smem > smem_limit()) break;
+            if (smem > cluster_smem_limit()) break;
             const int64_t groups = (b + cols - 1) / cols;
             const int act = active_clusters(pick_kernel<T>(!doubling, width, rpt, cg), size, threads, smem);
             if (act < 1) continue;
@@ -500,7 +456,7 @@ int cluster_batch_plan(const std::vector<int64_t> &rows_of, int width, int64_t b
                                     ClusterJob{(int)i, c0, std::min<int>(c, (int)b - c0), 0}});
             }
             const size_t smem = vec + sum_bytes(threads, cols, doubling);
-            if (smem > smem_limit()) break;
+            if (smem > cluster_smem_limit()) break;
             const int cg = cols == 1 ? 1 : 4;
             const int act = active_clusters(pick_kernel<T>(!doubling, width, rpt, cg), size, threads, smem);
             if (act < 1) continue;

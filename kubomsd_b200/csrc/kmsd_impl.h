@@ -235,6 +235,10 @@ struct kmsd_engine_s {
     // (complex, FP64 and FP32 copies); built on first use, -1: cannot align
     kmsd::DevBuf vell64[3], vell32[3];
     int vell_state[3] = {0, 0, 0};
+    // per axis, the entries of a purely imaginary explicit velocity in H's CSR
+    // order (kmsd_cluster_series.cu); built on first use, -1: it is not one
+    kmsd::DevBuf vcsr64[3], vcsr32[3];
+    int vcsr_state[3] = {0, 0, 0};
     kmsd::DevBuf status;  // int[4]: [0] code, [1] report claim, [2] series nonfinite
     kmsd::DevBuf report;  // FailReportFull
     kmsd::DevBuf dots;    // double2[512]

@@ -742,6 +742,80 @@ int compute_inj(E *e, const double2 *X, int64_t W, const Aug &g, const Ctl &c, c
     return KMSD_OK;
 }
 
+// The explicit velocity of axis x as imaginary values in H's CSR order; false
+// when it has a real part or an entry outside H's pattern.
+bool imaginary_velocity(E *e, int x) {
+    if (e->vcsr_state[x]) return e->vcsr_state[x] > 0;
+    e->vcsr_state[x] = -1;
+    const kmsd_csr_s *H = e->H, *V = e->vel[3 * x];
+    const int64_t n = H->n;
+    if (H->complex_values || !V || !V->complex_values || V->nnz < 1 || H->nnz < 1) return false;
+    std::vector<int> hp(n + 1), hi(H->nnz), vp(n + 1), vi(V->nnz);
+    std::vector<double> vr(V->nnz), vim(V->nnz), im(H->nnz, 0.);
+    if (cudaMemcpy(hp.data(), H->ptr, hp.size() * sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess ||
+        cudaMemcpy(hi.data(), H->idx, hi.size() * sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess ||
+        cudaMemcpy(vp.data(), V->ptr, vp.size() * sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess ||
+        cudaMemcpy(vi.data(), V->idx, vi.size() * sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess ||
+        cudaMemcpy(vr.data(), V->re64, vr.size() * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess ||
+        cudaMemcpy(vim.data(), V->im64, vim.size() * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess)
+        return false;
+    for (int64_t r = 0; r < n; ++r) {
+        int h = hp[r];  // V's entries in H's order, so that the sums run in V's own order
+        for (int k = vp[r]; k < vp[r + 1]; ++k) {
+            if (vr[k] != 0.) return false;
+            while (h < hp[r + 1] && hi[h] != vi[k]) ++h;
+            if (h == hp[r + 1]) return false;
+            im[h++] = vim[k];
+        }
+    }
+    const std::vector<float> im32(im.begin(), im.end());
+    if (e->vcsr64[x].ensure(im.size() * sizeof(double)) || e->vcsr32[x].ensure(im32.size() * sizeof(float))) return false;
+    if (cudaMemcpy(e->vcsr64[x].p, im.data(), im.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(e->vcsr32[x].p, im32.data(), im32.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess)
+        return false;
+    e->vcsr_state[x] = 1;
+    return true;
+}
+
+template <class T> const T *vcsr_of(E *e, int x);
+template <> const double *vcsr_of<double>(E *e, int x) { return e->vcsr64[x].as<double>(); }
+template <> const float *vcsr_of<float>(E *e, int x) { return e->vcsr32[x].as<float>(); }
+
+// A series of a small real operator on an orthogonal basis as one launch per
+// direction (kmsd_cluster_series.cu), each along one axis with a purely imaginary
+// explicit velocity; *done says whether that path took the call.
+template <class T>
+int series_small(E *e, const double2 *B, double2 *out, int64_t b, const double *coeff, int64_t nc, double center,
+                 double half, const Aug &g, cudaStream_t s, bool *done) {
+    *done = false;
+    if (!e->identity || e->H->complex_values || nc > kSeriesTerms) return KMSD_OK;
+    ClusterPlan pl;
+    if (int rc = series_plan<T>(e->H->n, e->H->row_max, g.nb, g.ndir > 0, &pl)) return rc;
+    if (!pl.size) return KMSD_OK;
+    int axis[3] = {0, 0, 0};
+    for (int64_t d = 0; d < g.ndir; ++d) {
+        int used = 0;
+        for (int x = 0; x < 3; ++x)
+            if (g.dirs[3 * d + x] != 0.) {
+                axis[d] = x;
+                ++used;
+            }
+        if (used != 1 || e->vel_kind[axis[d]] != 0 || !imaginary_velocity(e, axis[d])) return KMSD_OK;
+    }
+    if (std::is_same<T, float>::value && e->H->ensure_f32()) return KMSD_ECUDA;
+    for (int64_t d = 0; d < std::max<int64_t>(g.ndir, 1); ++d) {
+        const T *vim = g.ndir ? vcsr_of<T>(e, axis[d]) : nullptr;
+        const double wi = g.ndir ? -e->hbar / half * g.dirs[3 * d + axis[d]] : 0.;
+        if (int rc = cluster_series<T>(pl, view_of<T>(e->H), e->H->row_max, e->H->n, vim, wi, B, out, b, g.nb,
+                                       (d + 1) * g.nb, d + 1 >= g.ndir, coeff, nc, center, half, status_ptr(e) + 2, s))
+            return rc;
+    }
+    e->h_calls += nc - 1;
+    e->v_calls += (nc - 1) * g.ndir;
+    *done = true;
+    return KMSD_OK;
+}
+
 int series_impl(E *e, const double2 *B, double2 *out, int64_t b, const double *coeff, int64_t nc, double center,
                 double half, const double *dirs, int64_t ndir, cudaStream_t s) {
     const int64_t n = e->H->n;
@@ -757,6 +831,7 @@ int series_impl(E *e, const double2 *B, double2 *out, int64_t b, const double *c
     g.ndir = ndir;
     g.dirs = dirs;
     g.nb = ndir ? b / (ndir + 1) : b;
+    bool done = false;
     if (ndir && (rc = plan_aug(e, g))) return rc;
     if (e->precision == KMSD_MIXED) {
         if (!e->identity) return fail(KMSD_EINVAL, "mixed precision requires an identity metric (orthogonal basis)");
@@ -765,6 +840,7 @@ int series_impl(E *e, const double2 *B, double2 *out, int64_t b, const double *c
                                      "operator given by site coordinates (kind 1, diagonal)");
         if (ndir && g.nb % 2)
             return fail(KMSD_EINVAL, "mixed-precision propagation needs an even number of vectors per block");
+        if ((rc = series_small<float>(e, B, out, b, coeff, nc, center, half, g, s, &done)) || done) return rc;
         const int U = (int)((b + 1) / 2);
         if (ensure_vec(e->ta, n, U, sizeof(float4)) || ensure_vec(e->tb, n, U, sizeof(float4)) ||
             ensure_vec(e->outw, n, U, sizeof(float4)) || e->H->ensure_f32())
@@ -797,6 +873,7 @@ int series_impl(E *e, const double2 *B, double2 *out, int64_t b, const double *c
         e->v_calls += (nc - 1) * ndir;
         return to_f64(ow, out, n, b, U, s);
     }
+    if ((rc = series_small<double>(e, B, out, b, coeff, nc, center, half, g, s, &done)) || done) return rc;
     if (ensure_vec(e->ta, n, b) || ensure_vec(e->tb, n, b)) return KMSD_ECUDA;
     double2 *ta = e->ta.as<double2>(), *tb = e->tb.as<double2>();
     StepArgs<double> a = base_args<double>(e, (int)b, center, half);
@@ -900,7 +977,8 @@ void kmsd_engine_destroy(kmsd_engine e) {
     for (DevBuf *d : {&e->ta, &e->tb, &e->bra, &e->hx, &e->t1, &e->t2, &e->t3, &e->t4, &e->t5, &e->psi, &e->vc,
                       &e->inj[0], &e->inj[1], &e->inj[2], &e->outw, &e->status, &e->report, &e->dots, &e->cluster,
                       &e->ring, &e->corr_partial, &e->vell64[0], &e->vell64[1], &e->vell64[2], &e->vell32[0],
-                      &e->vell32[1], &e->vell32[2]})
+                      &e->vell32[1], &e->vell32[2], &e->vcsr64[0], &e->vcsr64[1], &e->vcsr64[2],
+                      &e->vcsr32[0], &e->vcsr32[1], &e->vcsr32[2]})
         d->release();
     e->red.partial.release();
     e->red.ticket.release();

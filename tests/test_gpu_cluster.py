@@ -93,3 +93,52 @@ def test_cluster_batch(cuda, sizes, b, M, precision, doubling):
         want = eng.moments(Bs[i], M, centers[i], halves[i], doubling=doubling)
         # the same elements, the FP64 sums in another order
         assert_rel(got[i], want, 1e-13, f"instance {i}")
+
+
+def velocity_of(H, seed, drop=0.):
+    """A purely imaginary Hermitian velocity on (part of) H's off-diagonal pattern."""
+    U = sp.triu(H, 1).tocoo()
+    rng = np.random.default_rng(seed)
+    w = rng.uniform(.2, 1., U.nnz) * (rng.random(U.nnz) >= drop)
+    A = sp.coo_matrix((1j * U.data * w, (U.row, U.col)), shape=H.shape).tocsr()
+    A.eliminate_zeros()
+    return (A + A.conj().T).tocsr()
+
+
+# rows, reach, psi columns, directions: shares of 480 / 608 rows and their doubles,
+# no phi block, one and two directions, one with a velocity outside one axis
+@pytest.mark.parametrize("n,reach,nb,dirs", [(7, 1, 2, [[1., 0., 0.]]), (480, 2, 4, [[1., 0., 0.]]), (4096, 2, 8, []),
+                                             (1000, 3, 6, [[1., 0., 0.], [0., -1., 0.]]), (9729, 2, 2, [[0., 2., 0.]]),
+                                             (15360, 2, 34, [[1., 0., 0.]]), (4096, 1, 2, [[.6, .8, 0.]])])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_cluster_series(cuda, n, reach, nb, dirs, precision):
+    from oracle import kpm_oracle as O
+    from tests.gpu_util import engine
+    H = ring(n, reach, n + nb)
+    V = {"x": velocity_of(H, 1), "y": velocity_of(H, 2, .5)}
+    S = sp.identity(n, format="csr")
+    half = 1.05 * float(abs(H).sum(axis=1).max()) + .1
+    rng = np.random.default_rng(n)
+    b = nb * (1 + len(dirs))
+    B = rng.standard_normal((n, b)) + 1j * rng.standard_normal((n, b))
+    _, eng, _ = engine(H, S, velocity=V, precision=precision)
+    ref = O.engine_from_model(H, S, velocity=V)
+    for terms in (2, 3, 40):
+        coeff = (rng.standard_normal(terms) + 1j * rng.standard_normal(terms)) * .8 ** np.arange(terms)
+        before = eng.lib.kmsd_kernel_launches()
+        got = eng.series(B, coeff, .03, half, dirs)
+        launches = eng.lib.kmsd_kernel_launches() - before
+        if all(np.count_nonzero(d) == 1 and V["xy"[np.argmax(np.abs(d))]].nnz for d in dirs):
+            assert launches == max(1, len(dirs))
+        assert_rel(got, ref.series(B, coeff, .03, half, dirs), 1e-10 if precision == "fp64" else 5e-5, f"{terms}")
+    assert eng.core.h_calls == 1 + 2 + 39 and eng.core.v_calls == 42 * len(dirs)
+
+
+def test_cluster_series_reports_nonfinite(cuda):
+    from kubomsd_b200.errors import NumericalError
+    from tests.gpu_util import engine
+    H = ring(300, 2, 9)
+    _, eng, _ = engine(H, sp.identity(300, format="csr"))
+    B = np.ones((300, 2), complex)
+    with pytest.raises(NumericalError, match="nonfinite Chebyshev propagation"):
+        eng.series(B, np.ones(150), 0., 1e-3)  # far outside the window: T_k overflows
