@@ -365,6 +365,11 @@ int kmsd_engine_inner(kmsd_engine e, const void *a, const void *b_in, void *out,
 int kmsd_column_dot(const void *x, const void *y, int64_t n, int64_t b,
                     void *out, void *stream);
 
+/* *finite = 1 when all `count` complex128 values of the device array x are
+ * finite, else 0 (the check of Dense(const Arr&), cpp/native.cpp:31-40).
+ * Synchronises the stream. */
+int kmsd_check_finite(const void *x, int64_t count, int *finite, void *stream);
+
 /* ---- Ragged batches (the batching form; no counterpart in the reference) */
 
 /* A batch of `ninst` independent orthogonal-basis Hamiltonians of any sizes,

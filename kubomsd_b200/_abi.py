@@ -79,6 +79,7 @@ SIGNATURES = {
     "kmsd_engine_counters": (C.c_int, [P, PI64, PI64]),
     "kmsd_engine_failure_report": (C.c_int, [P, C.POINTER(SolveReport), I64, PI64]),
     "kmsd_engine_inner": (C.c_int, [P, P, P, P, I64, P]),
+    "kmsd_check_finite": (C.c_int, [P, I64, C.POINTER(C.c_int), P]),
     "kmsd_column_dot": (C.c_int, [P, P, I64, I64, P, P]),
     "kmsd_batch_create": (C.c_int, [I64, C.POINTER(P), C.c_int, I64, C.POINTER(P)]),
     "kmsd_batch_attach_metric": (C.c_int, [P, P, P, D, D, C.c_int]),

@@ -503,6 +503,31 @@ int kmsd_csr_matmul(kmsd_csr a, const void *x, void *y, int64_t b, void *stream)
                   static_cast<cudaStream_t>(stream));
 }
 
+int kmsd_check_finite(const void *x, int64_t count, int *finite, void *stream) {
+    if (!x || !finite || count < 0 || (reinterpret_cast<uintptr_t>(x) & 15u))
+        return fail(KMSD_EINVAL, "invalid finiteness check");
+    // the flag is host memory that the device writes: nothing to copy back
+    struct Flag {
+        int *p = nullptr;
+        ~Flag() {
+            if (p) cudaFreeHost(p);
+        }
+    };
+    static thread_local Flag flag;
+    if (!flag.p) KMSD_CUDA(cudaHostAlloc((void **)&flag.p, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    *(volatile int *)flag.p = 0;
+    if (count > 0) {
+        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((count + 1023) / 1024, (int64_t)sm_count() * 8));
+        finite_scan_kernel<<<grid, 256, 0, s>>>(static_cast<const uint4 *>(x), count, flag.p);
+        count_launch();
+        KMSD_CUDA(cudaGetLastError());
+        KMSD_CUDA(cudaStreamSynchronize(s));
+    }
+    *finite = *(volatile int *)flag.p == 0;
+    return KMSD_OK;
+}
+
 int kmsd_column_dot(const void *x, const void *y, int64_t n, int64_t b, void *out, void *stream) {
     if (!x || !y || !out || n < 1 || b < 1) return fail(KMSD_EINVAL, "invalid column dot dimensions");
     return coldot64(static_cast<const double2 *>(x), static_cast<const double2 *>(y), n, b,

@@ -936,15 +936,24 @@ static __global__ void lincomb_kernel(Lincomb L, double2 *y, int64_t len) {
     }
 }
 
-// Nonfinite scan: status |= 1 if any element is nonfinite.
-static __global__ void finite_scan_kernel(const double2 *x, int64_t len, int *status) {
-    bool bad = false;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < len;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const double2 v = x[i];
-        bad |= !isfinite(v.x) || !isfinite(v.y);
+// *bad = 1 if any of `len` complex values is nonfinite (their exponent bits all
+// set).  One read of the array at HBM speed, four loads of a thread in flight.
+static __global__ void __launch_bounds__(256) finite_scan_kernel(const uint4 *x, int64_t len, int *bad) {
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    bool any = false;
+    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    auto check = [&](const uint4 &v) {
+        any |= (v.y & 0x7ff00000u) == 0x7ff00000u || (v.w & 0x7ff00000u) == 0x7ff00000u;
+    };
+    for (; i + 3 * step < len; i += 4 * step) {
+        uint4 v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = __ldg(x + i + q * step);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) check(v[q]);
     }
-    if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(status, 1);
+    for (; i < len; i += step) check(__ldg(x + i));
+    if (any) *(volatile int *)bad = 1;
 }
 
 }  // namespace kmsd

@@ -363,14 +363,16 @@ int moments_impl(E *e, const double2 *B, double *mu, int64_t b, int64_t len, dou
     if (done) return KMSD_OK;
     if (e->precision == KMSD_FP64) {
         const double2 *bra = B;
-        if (e->identity) {
+        const bool given = doubling && len > 1;  // the first step's sums are mu_0 and mu_1
+        if (given) {
+        } else if (e->identity) {
             if ((rc = coldot64(B, B, n, b, dots, s))) return rc;
         } else {
             if (ensure_vec(e->bra, n, b)) return KMSD_ECUDA;
             if ((rc = spmm64(e->M->S, B, e->bra.as<double2>(), b, s, dots))) return rc;
             bra = e->bra.as<double2>();
         }
-        if ((rc = take_real(dots, mu, b, s))) return rc;
+        if (!given && (rc = take_real(dots, mu, b, s))) return rc;
         if (len == 1) return KMSD_OK;
         if (ensure_vec(e->ta, n, b) || ensure_vec(e->tb, n, b)) return KMSD_ECUDA;
         double2 *ta = e->ta.as<double2>(), *tb = e->tb.as<double2>();
@@ -431,24 +433,26 @@ int moments_impl(E *e, const double2 *B, double *mu, int64_t b, int64_t len, dou
     // Mixed: identity metric only.
     if (!e->identity) return fail(KMSD_EINVAL, "mixed precision requires an identity metric (orthogonal basis)");
     const int U = (int)((b + 1) / 2);
+    // T_0 -> tb; direct moments keep it as their bra and rotate two other buffers
     if (ensure_vec(e->ta, n, U, sizeof(float4)) || ensure_vec(e->tb, n, U, sizeof(float4)) ||
-        ensure_vec(e->bra, n, U, sizeof(float4)) || e->H->ensure_f32())
+        (!doubling && ensure_vec(e->bra, n, U, sizeof(float4))) || e->H->ensure_f32())
         return KMSD_ECUDA;
-    float4 *ta = e->ta.as<float4>(), *tb = e->tb.as<float4>(), *bra = e->bra.as<float4>();
+    float4 *ta = e->ta.as<float4>(), *tb = e->tb.as<float4>();
     if ((rc = to_f32(B, tb, n, b, U, s))) return rc;
-    if (!doubling) KMSD_CUDA(cudaMemcpyAsync(bra, tb, (size_t)n * U * sizeof(float4), cudaMemcpyDeviceToDevice, s));
-    if ((rc = coldot32(tb, tb, n, U, dots, s))) return rc;
-    if ((rc = take_real(dots, mu, b, s))) return rc;
-    if (len == 1) return KMSD_OK;
+    if (!doubling || len == 1) {  // else the first step's sums are mu_0 and mu_1
+        if ((rc = coldot32(tb, tb, n, U, dots, s))) return rc;
+        if ((rc = take_real(dots, mu, b, s))) return rc;
+        if (len == 1) return KMSD_OK;
+    }
     StepArgs<float> a = base_args<float>(e, U, center, half);
-    a.bra = bra;
+    a.bra = tb;
     a.mu = mu;
     a.mlen = len;
     a.bcols = (int)b;
-    float4 *curr = tb, *prev = nullptr, *spare = ta;
+    float4 *curr = tb, *prev = nullptr, *spare = doubling ? nullptr : e->bra.as<float4>();
     const int64_t steps = doubling ? (len + 1) / 2 : len - 1;
     for (int64_t k = 1; k <= steps; ++k) {
-        float4 *next = k == 1 ? spare : prev;
+        float4 *next = k == 1 ? ta : k == 2 && spare ? spare : prev;
         a.curr = curr;
         a.prev = prev;
         a.next = next;
