@@ -7,14 +7,13 @@
 // T_k(Ht) v.  The left chain is generated into a ring of kRing vector blocks
 // by the engine's fused Chebyshev step; every kRing steps one contraction
 // launch reduces the ring against cov:
-//   * corr_partial_kernel: CTA (row chunk, tile of kJT chain vectors); each
-//     thread owns one column b and up to KPT values of k for all kJT chain
-//     vectors, and walks the rows of its chunk; partial sums per chunk;
-//   * corr_reduce_kernel: tables = sum over chunks in chunk order.
-// Row ownership and the chunk order are fixed, so the tables are the same in
-// every run.  HBM per ring: the ring written once by the steps and read once
-// here, and cov read once (the kRing / kJT tiles of a chunk are neighbouring
-// CTAs and meet cov in L2).
+//   * corr_partial_kernel: CTA (row chunk, tile of k); each thread owns one
+//     column b, 8 chain vectors and 4 values of k, and walks the rows of its
+//     chunk; partial sums per chunk;
+//   * corr_reduce_kernel: tables = sum over chunks in a fixed order.
+// Row ownership and the order of the sums are fixed, so the tables are the same
+// in every run.  HBM per ring: the ring written once by the steps and read once
+// here, and cov read once per k tile.
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -28,95 +27,138 @@ using namespace kmsd;
 namespace {
 
 constexpr int kRing = 32;  // left-chain vector blocks held at once
-constexpr int kJT = 8;     // chain vectors per contraction tile
-constexpr int kCorrThreads = 256;
+constexpr int kJT = 8;     // chain vectors of a thread
+constexpr int kKT = 4;     // right-chain terms of a thread
+constexpr int kJG = kRing / kJT;
+constexpr int kCorrThreads = 352;  // most threads of a CTA (184 registers each)
+constexpr int kStages = 3;
+
+__device__ __forceinline__ void copy16(void *smem, const void *global) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(global) : "memory");
+}
 
 // partial[chunk][jj][k][b] for the ring's chain vectors jj < jn (ring slot
 // (j0 + jj) % kRing), rows [chunk * rows_per, ...).
-template <int KPT>
-__global__ void __launch_bounds__(kCorrThreads) corr_partial_kernel(const double2 *ring, int64_t slab,
-                                                                   const double2 *cov, int64_t n, int nb, int nbp,
-                                                                   int k1, int64_t j0, int jn, int64_t rows_per,
-                                                                   int ntiles, double2 *partial) {
-    const int chunk = blockIdx.x / ntiles, tile = blockIdx.x % ntiles;
+//
+// The contraction is FP64-bound: 8 flops per (row, j, k, b), 1.4 GFLOP per ring
+// of 16,384 rows, 41 terms and 8 columns, 40 us at the measured 34 TFLOP/s.  A
+// CTA takes all 32 chain vectors of its rows, so that cov is read once; a thread
+// holds an 8 x 4 tile of sums (128 registers), which needs 12 operand loads for
+// 128 multiply-adds; the operands of the next `rs` rows come in with cp.async
+// while these are multiplied.  One thread per (k, 8 vectors) without staging, a
+// quarter of the vectors per CTA, took 282 us here; this takes 91.
+__global__ void __launch_bounds__(kCorrThreads, 1) corr_partial_kernel(const double2 *ring, int64_t slab,
+                                                                       const double2 *cov, int64_t n, int nb, int nbp,
+                                                                       int k1, int kw, int64_t j0, int jn,
+                                                                       int64_t rows_per, int ktiles, int rs,
+                                                                       double2 *partial) {
+    extern __shared__ __align__(16) double2 stage[];  // kStages x ([kRing][rs][nb], [rs][kw][nb])
+    const int chunk = blockIdx.x / ktiles, tile = blockIdx.x % ktiles;
     const int t = threadIdx.x;
-    const int b = t % nbp, kg = t / nbp, kgroups = kCorrThreads / nbp;
-    const int jt0 = tile * kJT;
+    // neighbouring lanes: columns, then terms, then chain vectors
+    const int kgroups = (kw + kKT - 1) / kKT;
+    const int b = t % nbp, kg = t / nbp % kgroups, jg = t / nbp / kgroups;
+    const int kbase = tile * kw, kn = min(kw, k1 - kbase);
+    const bool active = b < nb && jg * kJT < jn;
     const int64_t r0 = (int64_t)chunk * rows_per, r1 = min(n, r0 + rows_per);
-    double2 acc[kJT][KPT];
+    const int tsize = kRing * rs * nb, ssize = tsize + rs * kw * nb;
+    double2 acc[kJT][kKT];
 #pragma unroll
     for (int jj = 0; jj < kJT; ++jj)
 #pragma unroll
-        for (int i = 0; i < KPT; ++i) acc[jj][i] = make_double2(0., 0.);
-    const bool active = b < nb;
-    const double2 *slot[kJT];
+        for (int i = 0; i < kKT; ++i) acc[jj][i] = make_double2(0., 0.);
+    auto fetch = [&](int64_t r, int slot) {  // rows [r, r + rs) into a stage
+        if (r < r1) {
+            const int rows = (int)min((int64_t)rs, r1 - r), tn = rows * nb, cn = kn * nb;
+            double2 *ts = stage + (size_t)slot * ssize, *cs = ts + tsize;
+            for (int i = t; i < jn * tn; i += blockDim.x) {
+                const int jj = i / tn, x = i - jj * tn;
+                copy16(ts + jj * rs * nb + x, ring + (size_t)((j0 + jj) % kRing) * slab + r * nb + x);
+            }
+            for (int i = t; i < rows * cn; i += blockDim.x) {
+                const int row = i / cn, x = i - row * cn;
+                copy16(cs + row * kw * nb + x, cov + ((r + row) * k1 + kbase) * nb + x);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int q = 0; q < kStages - 1; ++q) fetch(r0 + (int64_t)q * rs, q);
+    int slot = 0;
+    for (int64_t r = r0; r < r1; r += rs) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+        __syncthreads();  // this stage is in, and the one before it has been read by all
+        fetch(r + (int64_t)(kStages - 1) * rs, (slot + kStages - 1) % kStages);
+        if (active) {
+            const int rows = (int)min((int64_t)rs, r1 - r);
+            const double2 *ts = stage + (size_t)slot * ssize + jg * kJT * rs * nb + b;
+            const double2 *cs = stage + (size_t)slot * ssize + tsize + kg * kKT * nb + b;
+            for (int row = 0; row < rows; ++row) {
+                double2 kv[kKT];
+#pragma unroll
+                for (int i = 0; i < kKT; ++i) kv[i] = cs[(row * kw + min(i, kn - 1 - kg * kKT)) * nb];
+#pragma unroll
+                for (int jj = 0; jj < kJT; ++jj) {
+                    const double2 cv = ts[(jj * rs + row) * nb];
+#pragma unroll
+                    for (int i = 0; i < kKT; ++i) {
+                        // conj(cv) * kv
+                        acc[jj][i].x = fma(cv.x, kv[i].x, fma(cv.y, kv[i].y, acc[jj][i].x));
+                        acc[jj][i].y = fma(cv.x, kv[i].y, fma(-cv.y, kv[i].x, acc[jj][i].y));
+                    }
+                }
+            }
+        }
+        slot = slot + 1 == kStages ? 0 : slot + 1;
+    }
+    if (!active) return;
+    double2 *out = partial + (size_t)chunk * kRing * k1 * nb;
 #pragma unroll
     for (int jj = 0; jj < kJT; ++jj) {
-        const int jr = jt0 + jj < jn ? jt0 + jj : jn - 1;  // (clamped: never accumulated)
-        slot[jj] = ring + (size_t)((j0 + jr) % kRing) * slab;
-    }
-    if (active) {
-        for (int64_t r = r0; r < r1; ++r) {
-            double2 cv[kJT], kv[KPT];
+        if (jg * kJT + jj >= jn) break;
 #pragma unroll
-            for (int jj = 0; jj < kJT; ++jj) cv[jj] = __ldg(slot[jj] + r * nb + b);
-#pragma unroll
-            for (int i = 0; i < KPT; ++i) {
-                const int k = kg + i * kgroups;
-                kv[i] = k < k1 ? __ldg(cov + (r * k1 + k) * nb + b) : make_double2(0., 0.);
-            }
-#pragma unroll
-            for (int jj = 0; jj < kJT; ++jj)
-#pragma unroll
-                for (int i = 0; i < KPT; ++i) {
-                    // conj(cv) * kv
-                    acc[jj][i].x = fma(cv[jj].x, kv[i].x, fma(cv[jj].y, kv[i].y, acc[jj][i].x));
-                    acc[jj][i].y = fma(cv[jj].x, kv[i].y, fma(-cv[jj].y, kv[i].x, acc[jj][i].y));
-                }
-        }
-        double2 *out = partial + (size_t)chunk * kRing * k1 * nb;
-#pragma unroll
-        for (int jj = 0; jj < kJT; ++jj) {
-            if (jt0 + jj >= jn) break;
-#pragma unroll
-            for (int i = 0; i < KPT; ++i) {
-                const int k = kg + i * kgroups;
-                if (k < k1) out[((size_t)(jt0 + jj) * k1 + k) * nb + b] = acc[jj][i];
-            }
+        for (int i = 0; i < kKT; ++i) {
+            const int k = kg * kKT + i;
+            if (k < kn) out[((size_t)(jg * kJT + jj) * k1 + kbase + k) * nb + b] = acc[jj][i];
         }
     }
 }
 
-// tables[b][j0 + jj][k] = sum over chunks (in chunk order) of partial.
-__global__ void corr_reduce_kernel(const double2 *partial, int nchunks, int jn, int k1, int nb, int64_t j0,
-                                   int64_t length, double2 *tables) {
+// tables[b][j0 + jj][k] = sum over chunks of partial: a CTA takes 32 elements,
+// eight threads each, which sum every eighth chunk; their sums are joined in
+// order.
+__global__ void __launch_bounds__(256) corr_reduce_kernel(const double2 *partial, int nchunks, int jn, int k1, int nb,
+                                                          int64_t j0, int64_t length, double2 *tables) {
+    __shared__ double2 part[8][32];
     const int64_t total = (int64_t)jn * k1 * nb;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-        const int b = (int)(e % nb);
-        const int64_t jk = e / nb;
-        const int k = (int)(jk % k1), jj = (int)(jk / k1);
-        double sx = 0., sy = 0.;
-        const size_t stride = (size_t)kRing * k1 * nb;
-        for (int c = 0; c < nchunks; ++c) {
-            const double2 v = partial[c * stride + ((size_t)jj * k1 + k) * nb + b];
-            sx += v.x;
-            sy += v.y;
+    const size_t stride = (size_t)kRing * k1 * nb;
+    const int x = threadIdx.x & 31, q = threadIdx.x >> 5;
+    for (int64_t e0 = blockIdx.x * (int64_t)32; e0 < total; e0 += (int64_t)gridDim.x * 32) {
+        const int64_t e = e0 + x;
+        double2 s = make_double2(0., 0.);
+        if (e < total) {
+#pragma unroll 4
+            for (int c = q; c < nchunks; c += 8) {
+                const double2 v = partial[c * stride + e];
+                s.x += v.x;
+                s.y += v.y;
+            }
         }
-        tables[((size_t)b * length + j0 + jj) * k1 + k] = make_double2(sx, sy);
+        part[q][x] = s;
+        __syncthreads();
+        if (q == 0 && e < total) {
+#pragma unroll
+            for (int i = 1; i < 8; ++i) {
+                s.x += part[i][x].x;
+                s.y += part[i][x].y;
+            }
+            const int b = (int)(e % nb);
+            const int64_t jk = e / nb;
+            const int k = (int)(jk % k1), jj = (int)(jk / k1);
+            tables[((size_t)b * length + j0 + jj) * k1 + k] = s;
+        }
+        __syncthreads();
     }
-}
-
-using PartialFn = void (*)(const double2 *, int64_t, const double2 *, int64_t, int, int, int, int64_t, int, int64_t,
-                           int, double2 *);
-
-PartialFn partial_kernel(int kpt) {
-    switch (kpt) {
-        case 1: return corr_partial_kernel<1>;
-        case 2: return corr_partial_kernel<2>;
-        case 3: return corr_partial_kernel<3>;
-        case 4: return corr_partial_kernel<4>;
-    }
-    return nullptr;
 }
 
 // ------------------------------------------------------------------ node tail
@@ -193,21 +235,28 @@ namespace kmsd {
 int corr_ring(const double2 *ring, int64_t n, int nb, const double2 *cov, int k1, int64_t j0, int jn,
               int64_t length, double2 *tables, DevBuf &partial, cudaStream_t s) {
     const int nbp = nb <= 1 ? 1 : nb <= 2 ? 2 : nb <= 4 ? 4 : 8;
-    const int kgroups = kCorrThreads / nbp;
-    const int kpt = (k1 + kgroups - 1) / kgroups;
-    const PartialFn fn = partial_kernel(kpt);
-    if (nb > 8 || fn == nullptr)
+    if (nb > 8 || k1 > 4 * (256 / nbp))
         return fail(KMSD_EINVAL, "correlation tables take at most 8 vectors and 1024/vectors right-chain terms per call");
-    const int ntiles = (jn + kJT - 1) / kJT;
-    int nchunks = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)sm_count() * 4 / ntiles, n));
+    // terms of a CTA: what its threads hold, shared evenly among the k tiles
+    const int most = kCorrThreads / (nbp * kJG) * kKT, ktiles = (k1 + most - 1) / most;
+    const int kw = (((k1 + ktiles - 1) / ktiles) + kKT - 1) / kKT * kKT;
+    const int threads = (nbp * kJG * (kw / kKT) + 31) / 32 * 32;
+    // rows of a stage: three stages in about 200 KB, at most 16 rows each
+    const size_t row_bytes = (size_t)(kRing + kw) * nb * sizeof(double2);
+    const int rs = (int)std::max<size_t>(1, std::min<size_t>(16, 200 * 1024 / kStages / row_bytes));
+    const size_t smem = kStages * rs * row_bytes;
+    int nchunks = (int)std::max<int64_t>(1, std::min<int64_t>(std::max(1, sm_count() / ktiles), (n + rs - 1) / rs));
     const int64_t rows_per = (n + nchunks - 1) / nchunks;
     nchunks = (int)((n + rows_per - 1) / rows_per);
     if (partial.ensure((size_t)nchunks * kRing * k1 * nb * sizeof(double2))) return KMSD_ECUDA;
-    fn<<<nchunks * ntiles, kCorrThreads, 0, s>>>(ring, n * nb, cov, n, nb, nbp, k1, j0, jn, rows_per, ntiles,
-                                                 partial.as<double2>());
+    static const cudaError_t attr = cudaFuncSetAttribute((const void *)corr_partial_kernel,
+                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    KMSD_CUDA(attr);
+    corr_partial_kernel<<<nchunks * ktiles, threads, smem, s>>>(ring, n * nb, cov, n, nb, nbp, k1, kw, j0, jn, rows_per,
+                                                                ktiles, rs, partial.as<double2>());
     count_launch();
     const int64_t total = (int64_t)jn * k1 * nb;
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, (int64_t)sm_count() * 8));
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((total + 31) / 32, (int64_t)sm_count() * 16));
     corr_reduce_kernel<<<grid, 256, 0, s>>>(partial.as<double2>(), nchunks, jn, k1, nb, j0, length, tables);
     count_launch();
     KMSD_CUDA(cudaGetLastError());
