@@ -65,6 +65,16 @@ __device__ __forceinline__ void doubling_sums(double &s0, double &s1, T xr, T xi
     }
 }
 
+// cmac_cplx for a purely imaginary value, term by term the same.
+template <class T>
+__device__ __forceinline__ void cmac_imag(Pk<T> &acc, T vi, const Pk<T> &x) {
+#pragma unroll
+    for (int c = 0; c < Pk<T>::C; ++c) {
+        acc.re[c] = fma(-vi, x.im[c], acc.re[c]);
+        acc.im[c] = fma(vi, x.re[c], acc.im[c]);
+    }
+}
+
 // acc[m] += sum_k A[row,k] X[k, unit u_m]   for the MU units of this lane.
 template <class T, int MU>
 __device__ __forceinline__ void gather_row(const CsrView<T> &A, const typename Unit<T>::vec *X,
@@ -388,7 +398,7 @@ template <class T> struct StepArgs {
     const double *xdiag[3];
     // vform[v] = 2: the velocity's values aligned with H's ELL columns
     // (vel_re/vel_im[row * w + j] pairs with H's ELL index [row * w + j]),
-    // applied from the ELL row the step already holds
+    // applied from the ELL row the step already holds; vel_re null: purely imaginary
     const T *vel_re[3], *vel_im[3];
     int nvel;              // number of velocity matrices in use
     int share_v;           // every velocity in use has vform 2: psi lanes share V psi (see gather_share_v)
@@ -526,14 +536,25 @@ __device__ __forceinline__ void gather_share_v(const StepArgs<T> &a, const EllRo
 #pragma unroll 1
     for (int v = 0; v < a.nvel; ++v) {
         Pk<T> vp = pk_zero<T>();
-        const T *vr = a.vel_re[v] + row * (4 * PF), *vi = a.vel_im[v] + row * (4 * PF);
+        const T *vr = a.vel_re[v], *vi = a.vel_im[v] + row * (4 * PF);
+        if (vr == nullptr) {
 #pragma unroll
-        for (int q = 0; q < PF; ++q) {
-            T r4[4], i4[4];
-            ld4(vr + 4 * q, r4);
-            ld4(vi + 4 * q, i4);
+            for (int q = 0; q < PF; ++q) {
+                T i4[4];
+                ld4(vi + 4 * q, i4);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) cmac_cplx(vp, r4[j], i4[j], xs[q][j]);
+                for (int j = 0; j < 4; ++j) cmac_imag(vp, i4[j], xs[q][j]);
+            }
+        } else {
+            vr += row * (4 * PF);
+#pragma unroll
+            for (int q = 0; q < PF; ++q) {
+                T r4[4], i4[4];
+                ld4(vr + 4 * q, r4);
+                ld4(vi + 4 * q, i4);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) cmac_cplx(vp, r4[j], i4[j], xs[q][j]);
+            }
         }
         st(slot + (size_t)v * blockDim.x, vp);
     }
@@ -709,11 +730,12 @@ __global__ void __launch_bounds__(256, (step_pairs<T, MU, MODE, HSRC>() ? KMSD_S
                             vp = ld(vshare + ((size_t)parity * a.nvel + v) * blockDim.x + g * mp.G + upsi);
                         } else if ((HSRC == HSRC_ELL4 || HSRC == HSRC_ELL8) && a.vform[v] == 2) {
                             vp = pk_zero<T>();
-                            const T *vr = a.vel_re[v] + row * (4 * PF), *vi = a.vel_im[v] + row * (4 * PF);
+                            const T *vr = a.vel_re[v] ? a.vel_re[v] + row * (4 * PF) : nullptr,
+                                    *vi = a.vel_im[v] + row * (4 * PF);
 #pragma unroll
                             for (int q = 0; q < PF; ++q) {
-                                T r4[4], i4[4];
-                                ld4(vr + 4 * q, r4);
+                                T r4[4] = {T(0), T(0), T(0), T(0)}, i4[4];
+                                if (vr) ld4(vr + 4 * q, r4);
                                 ld4(vi + 4 * q, i4);
                                 const int col[4] = {cur.idx[q].x, cur.idx[q].y, cur.idx[q].z, cur.idx[q].w};
 #pragma unroll

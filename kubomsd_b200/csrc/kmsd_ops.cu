@@ -688,7 +688,8 @@ bool aligned_velocity(E *e, int x) {
         cudaMemcpy(d32, re32.data(), m * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(d32 + m, im32.data(), m * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess)
         return false;
-    e->vell_state[x] = 1;
+    // 2: purely imaginary (the lattice velocities), the real plane is not read
+    e->vell_state[x] = std::all_of(re.begin(), re.end(), [](double v) { return v == 0.; }) ? 2 : 1;
     return true;
 }
 
@@ -707,7 +708,7 @@ template <class T> void set_inline_v(E *e, StepArgs<T> &a, const Aug &g, double 
         if (!comm) a.Vm[v] = view_of<T>(e->vel[3 * x]);
         if (aligned) {
             const size_t m = (size_t)e->H->n * e->H->ell_w;
-            a.vel_re[v] = vell_of<T>(e, x);
+            a.vel_re[v] = e->vell_state[x] == 2 ? nullptr : vell_of<T>(e, x);
             a.vel_im[v] = vell_of<T>(e, x) + m;
         }
         a.vel_axis[v] = x;
