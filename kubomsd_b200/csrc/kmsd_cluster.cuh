@@ -112,4 +112,13 @@ int cluster_series(const ClusterPlan &pl, const CsrView<T> &H, int width, int64_
                    const double2 *B, double2 *out, int64_t b, int64_t nb, int64_t phi0, bool write_psi,
                    const double *coeff, int64_t ncoeff, double center, double half, int *status, cudaStream_t s);
 
+// How a stored chain of b columns is computed.
+template <class T> int chain_plan(int64_t n, int width, int64_t b, ClusterPlan *out);
+// Queues T_k for k0 <= k < k1 from cur = T_{k0-1} and prev = T_{k0-2} (nullptr:
+// k0 is 1), all (n, b) complex128, into store + (ring ? k % ring : k) * n * b; cur
+// and prev may be blocks of that ring.
+template <class T>
+int cluster_chain(const ClusterPlan &pl, const CsrView<T> &H, int width, int64_t n, const double2 *cur, const double2 *prev,
+                  double2 *store, int ring, int64_t b, int64_t k0, int64_t k1, double center, double half, cudaStream_t s);
+
 }  // namespace kmsd

@@ -1,4 +1,7 @@
-// The Bessel series of small orthogonal-basis operators in one launch: the
+// The Bessel series and stored Chebyshev chains of small orthogonal-basis
+// operators in one launch.
+//
+// Series: the
 // propagation sum_k c_k T_k(A) of psi columns, alone or with the phi block of one
 // direction whose velocity is purely imaginary (the lattice velocities i H_ij
 // dx_ij / hbar).
@@ -188,6 +191,143 @@ __global__ void __launch_bounds__(kMaxCompute<T>, 1) cluster_series_kernel(const
     if (bad) atomicOr(a.status, 1);
 }
 
+template <class T> struct ChainArgs {
+    CsrView<T> H;
+    const double2 *cur, *prev;  // T_{k0-1}, T_{k0-2} (nullptr: k0 is 1)
+    double2 *store;             // T_k goes to store + (ring ? k % ring : k) * n * b
+    int64_t n, b;
+    int ring, cols;
+    int64_t k0, k1;
+    double center, half;
+};
+
+// T_k for k0 <= k < k1, every one stored.  The stores are issued between the two
+// halves of the meeting, so that the next arrival finds them under way for a
+// step (a meeting right behind global stores takes four times as long).
+template <class T, int W, int RPT>
+__global__ void __launch_bounds__(kMaxCompute<T>, 1) cluster_chain_kernel(const ChainArgs<T> a) {
+    using V = typename Cx<T>::type;
+    extern __shared__ __align__(16) unsigned char sm[];
+    unsigned rank, size;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
+    const int c0 = (int)(blockIdx.x / size) * a.cols, cols = min(a.cols, (int)(a.b - c0));
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, compute = blockDim.x;
+    const int rows = (int)((a.n + size - 1) / size);
+    const int mine = max(0, min(rows, (int)(a.n - (int64_t)rank * rows)));
+    const int cwarps = compute / 32, wr = max(1, (rows + 31) / 32), sets = column_sets(cwarps, rows);
+    const int set = sets > 1 ? warp / wr : 0, own = sets > 1 ? warp - set * wr : warp;
+    const int at_row = own * 32 + lane;
+    const bool works = set < sets && own < min(cwarps, (mine + 31) / 32) && set < cols;
+    // [T_{k-1} | T_k][column][row]
+    const unsigned plane = (unsigned)rows * sizeof(V), block = plane * cols;
+    const unsigned base = (unsigned)__cvta_generic_to_shared(sm);
+    V *vec = reinterpret_cast<V *>(sm);
+    const int64_t g0 = (int64_t)rank * rows;
+
+    unsigned at[RPT][W];
+    T val[RPT][W];
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+        const int r = i * compute + at_row;
+        const bool on = works && r < mine;
+        const int k0 = on ? a.H.ptr[g0 + r] : 0, k1 = on ? a.H.ptr[g0 + r + 1] : 0;
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+            at[i][j] = base + (on ? (unsigned)r * (unsigned)sizeof(V) : 0u);
+            val[i][j] = T(0);
+            if (k0 + j < k1) {
+                const int c = a.H.idx[k0 + j], owner = c / rows, loc = c - owner * rows;
+                val[i][j] = a.H.re[k0 + j];
+                at[i][j] = base + (unsigned)loc * (unsigned)sizeof(V);
+                if (owner != (int)rank) at[i][j] = remote_address(at[i][j], owner);
+            }
+        }
+    }
+    for (int i = tid; i < mine * cols; i += blockDim.x) {
+        const int r = i / cols, c = i - r * cols;
+        const int64_t g = (g0 + r) * a.b + c0 + c;
+        const double2 x = a.cur[g], p = a.prev ? a.prev[g] : make_double2(0., 0.);
+        V w;
+        w.x = (T)x.x;
+        w.y = (T)x.y;
+        vec[(size_t)c * rows + r] = w;
+        w.x = (T)p.x;
+        w.y = (T)p.y;
+        vec[(size_t)(cols + c) * rows + r] = w;
+    }
+    cluster_sync_all();
+
+    const T cen = (T)a.center, hal = (T)a.half, inv = (T)(1. / a.half);
+    unsigned cur = 0;
+    T two = a.prev ? T(2) : T(1);
+    for (int64_t k = a.k0; k < a.k1; ++k) {
+        const unsigned nxt = block - cur;
+        if (works) {
+            for (int c = set; c < cols; c += sets) {
+#pragma unroll
+                for (int i = 0; i < RPT; ++i) {
+                    const int r = i * compute + at_row;
+                    if (r < mine) {
+                        const unsigned off = (unsigned)c * plane, me = off + (unsigned)r * (unsigned)sizeof(V);
+                        V xv[W];
+#pragma unroll
+                        for (int j = 0; j < W; ++j) xv[j] = load_any(at[i][j] + off + cur, V{});
+                        const V x = *reinterpret_cast<const V *>(sm + me + cur);
+                        V *dst = reinterpret_cast<V *>(sm + me + nxt);
+                        const V pv = *dst;
+                        V h;
+                        h.x = h.y = T(0);
+#pragma unroll
+                        for (int j = 0; j < W; ++j) {
+                            h.x = fma(val[i][j], xv[j].x, h.x);
+                            h.y = fma(val[i][j], xv[j].y, h.y);
+                        }
+                        const T tr = rdiv(h.x - cen * x.x, hal, inv), ti = rdiv(h.y - cen * x.y, hal, inv);
+                        V nx;
+                        nx.x = fma(two, tr, -pv.x);
+                        nx.y = fma(two, ti, -pv.y);
+                        *dst = nx;
+                    }
+                }
+            }
+        }
+        cluster_arrive();
+        if (works) {
+            double2 *out = a.store + (size_t)(a.ring ? k % a.ring : k) * a.n * a.b;
+            for (int c = set; c < cols; c += sets)
+#pragma unroll
+                for (int i = 0; i < RPT; ++i) {
+                    const int r = i * compute + at_row;
+                    if (r < mine) {
+                        const V v = *reinterpret_cast<const V *>(sm + (unsigned)c * plane + (unsigned)r * (unsigned)sizeof(V) + nxt);
+                        out[(g0 + r) * a.b + c0 + c] = make_double2((double)v.x, (double)v.y);
+                    }
+                }
+        }
+        cluster_wait();
+        cur = nxt;
+        two = T(2);
+    }
+}
+
+template <class T, int W>
+const void *pick_chain_rows(int rpt) {
+    switch (rpt) {
+        case 1: return (const void *)cluster_chain_kernel<T, W, 1>;
+        case 2: return (const void *)cluster_chain_kernel<T, W, 2>;
+        case 3:
+            if constexpr (W < kClusterWidth) return (const void *)cluster_chain_kernel<T, W, 3>;
+    }
+    return nullptr;
+}
+template <class T>
+const void *pick_chain(int width, int rpt) {
+    if (width <= 4) return pick_chain_rows<T, 4>(rpt);
+    if (width <= 5) return pick_chain_rows<T, 5>(rpt);
+    return pick_chain_rows<T, 8>(rpt);
+}
+
 template <class T, int W, bool PHI>
 const void *pick_rows(int rpt) {
     switch (rpt) {
@@ -209,16 +349,17 @@ const void *pick_kernel(int width, int rpt, bool phi) {
     return phi ? pick_width<T, true>(width, rpt) : pick_width<T, false>(width, rpt);
 }
 
-}  // namespace
+enum { kChain = 0, kPsi = 1, kPsiPhi = 2 };
 
-namespace kmsd {
-
-template <class T> int series_plan(int64_t n, int width, int64_t nb, bool phi, ClusterPlan *out) {
+// The cheapest shape for nb (psi) columns of `what`, as the moments' plan with
+// the accumulator and the phi block (cached).
+template <class T> int find_plan(int what, int64_t n, int width, int64_t nb, ClusterPlan *out) {
     *out = ClusterPlan{};
     if (width < 1 || width > kClusterWidth) return KMSD_OK;
     static std::mutex lock;
-    static std::map<std::tuple<int64_t, int, int64_t, bool>, ClusterPlan> cache;
-    const auto key = std::make_tuple(n, width, nb, phi);
+    static std::map<std::tuple<int, int64_t, int, int64_t>, ClusterPlan> cache;
+    const auto key = std::make_tuple(what, n, width, nb);
+    const int planes = what == kChain ? 2 : what == kPsi ? 3 : 6, blocks = what == kPsiPhi ? 2 : 1;
     {
         std::lock_guard<std::mutex> guard(lock);
         const auto it = cache.find(key);
@@ -231,18 +372,17 @@ template <class T> int series_plan(int64_t n, int width, int64_t nb, bool phi, C
     for (int size : {16, 8, 4, 2, 1}) {
         const int64_t rows = (n + size - 1) / size;
         const int rpt = (int)((rows + kMaxCompute<T> - 1) / kMaxCompute<T>);
-        const void *kernel = pick_kernel<T>(width, rpt, phi);
+        const void *kernel = what == kChain ? pick_chain<T>(width, rpt) : pick_kernel<T>(width, rpt, what == kPsiPhi);
         if (!kernel) continue;
         const int threads = (int)(((rows + rpt - 1) / rpt + 31) / 32 * 32), warps = threads / 32;
         const int sets = column_sets(warps, (int)rows);
         for (int cols = 1; cols <= std::min<int64_t>(nb, 32); ++cols) {
-            const size_t smem = (size_t)rows * cols * 2 * sizeof(T) * 3 * (phi ? 2 : 1);
+            const size_t smem = (size_t)rows * cols * 2 * sizeof(T) * planes;
             if (smem > cluster_smem_limit()) break;
             const int64_t groups = (nb + cols - 1) / cols;
             const int act = active_clusters(kernel, size, threads, smem);
             if (act < 1) continue;
-            // as the moments' cost, with the accumulator and the phi block
-            const int64_t items = (int64_t)((cols + sets - 1) / sets) * rpt * (phi ? 2 : 1);
+            const int64_t items = (int64_t)((cols + sets - 1) / sets) * rpt * blocks;
             const double traffic = std::min<int64_t>(warps, sets * ((rows + 31) / 32)) * (width + 5.) * (2 * sizeof(T)) * 32 / 128.;
             const double cost = ((size > 1 ? 1000. : 600.) + items * std::max(400., traffic)) * ((groups + act - 1) / act);
             if (out->size == 0 || cost < best) {
@@ -254,6 +394,31 @@ template <class T> int series_plan(int64_t n, int width, int64_t nb, bool phi, C
     std::lock_guard<std::mutex> guard(lock);
     if (cache.size() >= 1024) cache.clear();
     cache[key] = *out;
+    return KMSD_OK;
+}
+
+}  // namespace
+
+namespace kmsd {
+
+template <class T> int series_plan(int64_t n, int width, int64_t nb, bool phi, ClusterPlan *out) {
+    return find_plan<T>(phi ? kPsiPhi : kPsi, n, width, nb, out);
+}
+template <class T> int chain_plan(int64_t n, int width, int64_t b, ClusterPlan *out) {
+    return find_plan<T>(kChain, n, width, b, out);
+}
+
+template <class T>
+int cluster_chain(const ClusterPlan &pl, const CsrView<T> &H, int width, int64_t n, const double2 *cur, const double2 *prev,
+                  double2 *store, int ring, int64_t b, int64_t k0, int64_t k1, double center, double half, cudaStream_t s) {
+    ChainArgs<T> a{H, cur, prev, store, n, b, ring, pl.cols, k0, k1, center, half};
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    cluster_config(cfg, at, pl.groups * pl.size, pl.size, pl.threads, pl.smem);
+    cfg.stream = s;
+    void *args[] = {&a};
+    KMSD_CUDA(cudaLaunchKernelExC(&cfg, pick_chain<T>(width, pl.rpt), args));
+    count_launch();
     return KMSD_OK;
 }
 
@@ -291,6 +456,10 @@ int cluster_series(const ClusterPlan &pl, const CsrView<T> &H, int width, int64_
 
 #define KMSD_SERIES_INSTANCES(T)                                                                                        \
     template int series_plan<T>(int64_t, int, int64_t, bool, ClusterPlan *);                                           \
+    template int chain_plan<T>(int64_t, int, int64_t, ClusterPlan *);                                                  \
+    template int cluster_chain<T>(const ClusterPlan &, const CsrView<T> &, int, int64_t, const double2 *,              \
+                                  const double2 *, double2 *, int, int64_t, int64_t, int64_t, double, double,          \
+                                  cudaStream_t);                                                                       \
     template int cluster_series<T>(const ClusterPlan &, const CsrView<T> &, int, int64_t, const T *, double,           \
                                    const double2 *, double2 *, int64_t, int64_t, int64_t, bool, const double *,        \
                                    int64_t, double, double, int *, cudaStream_t);

@@ -472,6 +472,28 @@ int moments_impl(E *e, const double2 *B, double *mu, int64_t b, int64_t len, dou
 }
 
 // ---------------------------------------------------------------- chain
+// Steps k0 <= k < k1 of the chain of a small real operator on an orthogonal basis
+// as one launch (kmsd_cluster_series.cu), T_k into store + (ring ? k % ring : k)
+// blocks, where T_{k0-1} and T_{k0-2} are; *done says whether that path took them.
+template <class T>
+int chain_small(E *e, double2 *store, int ring, int64_t b, int64_t k0, int64_t k1, double center, double half,
+                cudaStream_t s, bool *done) {
+    *done = false;
+    if (!e->identity || e->H->complex_values) return KMSD_OK;
+    const int64_t slab = e->H->n * b;
+    ClusterPlan pl;
+    if (int rc = chain_plan<T>(e->H->n, e->H->row_max, b, &pl)) return rc;
+    if (!pl.size) return KMSD_OK;
+    if (std::is_same<T, float>::value && e->H->ensure_f32()) return KMSD_ECUDA;
+    auto at = [&](int64_t k) { return store + (ring ? k % ring : k) * slab; };
+    const int rc = cluster_chain<T>(pl, view_of<T>(e->H), e->H->row_max, e->H->n, at(k0 - 1), k0 >= 2 ? at(k0 - 2) : nullptr,
+                                    store, ring, b, k0, k1, center, half, s);
+    if (rc) return rc;
+    e->h_calls += k1 - k0;
+    *done = true;
+    return KMSD_OK;
+}
+
 int chain_impl(E *e, const double2 *B, double2 *out, int64_t b, int64_t len, double center, double half,
                cudaStream_t s) {
     const int64_t n = e->H->n;
@@ -480,7 +502,9 @@ int chain_impl(E *e, const double2 *B, double2 *out, int64_t b, int64_t len, dou
     int rc;
     KMSD_CUDA(cudaMemcpyAsync(out, B, slab * sizeof(double2), cudaMemcpyDeviceToDevice, s));
     if (len == 1) return KMSD_OK;
+    bool done = false;
     if (e->precision == KMSD_FP64) {
+        if ((rc = chain_small<double>(e, out, 0, b, 1, len, center, half, s, &done)) || done) return rc;
         StepArgs<double> a = base_args<double>(e, (int)b, center, half);
         if (!e->identity) {
             if (ensure_vec(e->hx, n, b)) return KMSD_ECUDA;
@@ -503,6 +527,7 @@ int chain_impl(E *e, const double2 *B, double2 *out, int64_t b, int64_t len, dou
     }
     if (!e->identity) return fail(KMSD_EINVAL, "mixed precision requires an identity metric (orthogonal basis)");
     if (b % 2) return fail(KMSD_EINVAL, "mixed-precision chain needs an even number of columns");
+    if ((rc = chain_small<float>(e, out, 0, b, 1, len, center, half, s, &done)) || done) return rc;
     const int U = (int)(b / 2);
     if (ensure_vec(e->ta, n, U, sizeof(float4)) || ensure_vec(e->tb, n, U, sizeof(float4)) || e->H->ensure_f32())
         return KMSD_ECUDA;
@@ -549,7 +574,21 @@ int correlate_impl(E *e, const double2 *B, const double2 *cov, int64_t b, int64_
     KMSD_CUDA(cudaMemcpyAsync(slot(0), B, slab * sizeof(double2), cudaMemcpyDeviceToDevice, s));
     if ((rc = contract_after(0))) return rc;
     if (len == 1) return KMSD_OK;
+    // small operators: the steps up to the ring's next contraction in one launch
+    auto small = [&](auto real, bool *done) -> int {
+        using T = decltype(real);
+        for (int64_t k = 1; k < len;) {
+            const int64_t end = std::min<int64_t>(len, k - k % J + J);
+            const int rc = chain_small<T>(e, ring, J, b, k, end, center, half, s, done);
+            if (rc || !*done) return rc;
+            if (int rc2 = contract_after(end - 1)) return rc2;
+            k = end;
+        }
+        return KMSD_OK;
+    };
+    bool done = false;
     if (e->precision == KMSD_FP64) {
+        if ((rc = small(double(), &done)) || done) return rc;
         StepArgs<double> a = base_args<double>(e, (int)b, center, half);
         if (!e->identity) {
             if (ensure_vec(e->hx, n, b)) return KMSD_ECUDA;
@@ -573,6 +612,7 @@ int correlate_impl(E *e, const double2 *B, const double2 *cov, int64_t b, int64_
     }
     if (!e->identity) return fail(KMSD_EINVAL, "mixed precision requires an identity metric (orthogonal basis)");
     if (b % 2) return fail(KMSD_EINVAL, "mixed-precision chain needs an even number of columns");
+    if ((rc = small(float(), &done)) || done) return rc;
     const int U = (int)(b / 2);
     if (ensure_vec(e->ta, n, U, sizeof(float4)) || ensure_vec(e->tb, n, U, sizeof(float4)) || e->H->ensure_f32())
         return KMSD_ECUDA;

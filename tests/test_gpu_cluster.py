@@ -142,3 +142,24 @@ def test_cluster_series_reports_nonfinite(cuda):
     B = np.ones((300, 2), complex)
     with pytest.raises(NumericalError, match="nonfinite Chebyshev propagation"):
         eng.series(B, np.ones(150), 0., 1e-3)  # far outside the window: T_k overflows
+
+
+@pytest.mark.parametrize("n,reach,b,length", [(7, 1, 2, 2), (480, 2, 4, 33), (3000, 3, 6, 5), (15361, 1, 2, 4), (1000, 2, 34, 3)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_cluster_chain(cuda, n, reach, b, length, precision):
+    from oracle import kpm_oracle as O
+    from tests.gpu_util import engine
+    H = ring(n, reach, n + b)
+    S = sp.identity(n, format="csr")
+    half = 1.05 * float(abs(H).sum(axis=1).max()) + .1
+    rng = np.random.default_rng(n)
+    B = rng.standard_normal((n, b)) + 1j * rng.standard_normal((n, b))
+    _, eng, _ = engine(H, S, precision=precision)
+    got = eng.chain(B, length, .03, half)
+    assert_rel(got, O.engine_from_model(H, S).chain(B, length, .03, half), 1e-10 if precision == "fp64" else 5e-5)
+    assert eng.core.h_calls == length - 1
+    # the same chain through the ring of the correlation tables, against cov = B
+    cov = np.ascontiguousarray(np.broadcast_to(B[:, None, :], (n, 1, b)))
+    tables = eng.chain_correlate(B, cov, length, .03, half).cpu().numpy()[:, :, 0]
+    want = np.einsum("jnb,nb->bj", got.conj(), B)
+    assert np.all(abs(tables - want) <= 1e-12 * np.einsum("jnb,nb->bj", abs(got), abs(B)))
