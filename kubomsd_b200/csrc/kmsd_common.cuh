@@ -295,6 +295,7 @@ __device__ __forceinline__ void final_column_sums(const double2 *partial, int np
         __syncthreads();
         if (threadIdx.x < cols) {
             double tx = 0., ty = 0.;
+#pragma unroll 8
             for (int p = 0; p < split; ++p) {
                 const double2 v = smem[p * cols + threadIdx.x];
                 tx += v.x;

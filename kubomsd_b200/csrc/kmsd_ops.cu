@@ -160,7 +160,7 @@ int launch_step_mu(E *e, StepArgs<T> &a, cudaStream_t s) {
         sm = std::max(sm, (size_t)2 * a.nvel * kThreads * sizeof(typename Unit<T>::vec));
     const int grid = wave_grid((const void *)kern, sm, a.n, a.mp);
     if (MODE == MODE_DIRECT || MODE == MODE_DOUBLING) {
-        if (e->red.ensure(grid, a.mp.U * Unit<T>::C, 2)) return KMSD_ECUDA;
+        if (e->red.ensure(grid, a.mp.U * Unit<T>::C)) return KMSD_ECUDA;
         a.partial = e->red.part();
         a.ticket = e->red.tick();
     }
@@ -216,7 +216,7 @@ int launch_tile(E *e, StepArgs<T> &a, cudaStream_t s) {
     guard.unlock();
     const int64_t ntiles = (a.n + tr - 1) / tr;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)sm_count() * per_sm));
-    if (e->red.ensure(grid, mp.U * Unit<T>::C, 2)) return KMSD_ECUDA;
+    if (e->red.ensure(grid, mp.U * Unit<T>::C)) return KMSD_ECUDA;
     a.partial = e->red.part();
     a.ticket = e->red.tick();
     kern<<<grid, kTileThreads, sm, s>>>(a, L, status_ptr(e) + 3);

@@ -157,7 +157,7 @@ __host__ __device__ inline TileLayout tile_layout(int tr, int U, int w, int nvec
 // scratch if that is larger.
 __host__ inline size_t tile_smem(const TileLayout &L, const RowMap &mp, int C) {
     const size_t ring = (size_t)L.sbytes * KMSD_TILE_STAGES;
-    const size_t red = ((size_t)mp.gpc * mp.U * C + kTileThreads + 2 * 512) * sizeof(double2);
+    const size_t red = ((size_t)mp.gpc * mp.U * C + kTileThreads + 512) * sizeof(double2);
     return ring > red ? ring : red;
 }
 
@@ -188,12 +188,9 @@ __global__ void __launch_bounds__(kTileThreads, KMSD_TILE_MINB)
     __syncthreads();
     const int64_t ntiles = (n + TR - 1) / TR;
     const int64_t mine = (int64_t)blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-    double2 acc0[1][C], acc1[1][C];
+    double2 acc[1][C];  // (direct, -) or (even, odd)
 #pragma unroll
-    for (int c = 0; c < C; ++c) {
-        acc0[0][c] = make_double2(0., 0.);
-        acc1[0][c] = make_double2(0., 0.);
-    }
+    for (int c = 0; c < C; ++c) acc[0][c] = make_double2(0., 0.);
     if (tid >= kTileConsumers) {
         // ---------------------------------------------------------- producer
         if (tid == kTileConsumers) {
@@ -315,12 +312,12 @@ __global__ void __launch_bounds__(kTileThreads, KMSD_TILE_MINB)
                             const Pk<T> br = ld(bs + rr * U + u);
 #pragma unroll
                             for (int c = 0; c < C; ++c)
-                                acc0[0][c].x += (double)br.re[c] * (double)nx.re[c] +
+                                acc[0][c].x += (double)br.re[c] * (double)nx.re[c] +
                                                 (double)br.im[c] * (double)nx.im[c];
                         } else {
 #pragma unroll
                             for (int c = 0; c < C; ++c)
-                                doubling_sums<T>(acc0[0][c].x, acc1[0][c].x, x.re[c], x.im[c], nx.re[c], nx.im[c], a.exact_sums);
+                                doubling_sums<T>(acc[0][c].x, acc[0][c].y, x.re[c], x.im[c], nx.re[c], nx.im[c], a.exact_sums);
                         }
                     }
                 }
@@ -335,31 +332,11 @@ __global__ void __launch_bounds__(kTileThreads, KMSD_TILE_MINB)
     double2 *red = reinterpret_cast<double2 *>(tsm);
     double2 *tot = red + (size_t)mp.gpc * U * C;
     double2 *outbuf = tot + kTileThreads;
-    double *even = reinterpret_cast<double *>(outbuf + 512);
-    cta_column_sums<1, C>(acc0, mp, ncol, red, a.partial);
-    if (MODE == MODE_DOUBLING) cta_column_sums<1, C>(acc1, mp, ncol, red, a.partial + (size_t)gridDim.x * ncol);
+    cta_column_sums<1, C>(acc, mp, ncol, red, a.partial);
     if (!last_cta(a.ticket)) return;
     final_column_sums(a.partial, gridDim.x, ncol, tot, outbuf);
-    if (MODE == MODE_DIRECT) {
-        for (int j = threadIdx.x; j < a.bcols; j += blockDim.x) a.mu[(size_t)a.kmom * a.bcols + j] = outbuf[j].x;
-        return;
-    }
     __syncthreads();
-    for (int j = threadIdx.x; j < ncol; j += blockDim.x) even[j] = outbuf[j].x;
-    __syncthreads();
-    final_column_sums(a.partial + (size_t)gridDim.x * ncol, gridDim.x, ncol, tot, outbuf);
-    const int64_t nn = a.kmom;
-    for (int j = threadIdx.x; j < a.bcols; j += blockDim.x) {
-        const double se = even[j], so = outbuf[j].x;
-        if (nn == 0) {
-            a.mu[j] = se;
-            if (a.mlen > 1) a.mu[(size_t)a.bcols + j] = so;
-        } else {
-            const double mu0 = a.mu[j], mu1 = a.mu[(size_t)a.bcols + j];
-            if (2 * nn < a.mlen) a.mu[(size_t)(2 * nn) * a.bcols + j] = 2. * se - mu0;
-            if (2 * nn + 1 < a.mlen) a.mu[(size_t)(2 * nn + 1) * a.bcols + j] = 2. * so - mu1;
-        }
-    }
+    store_moments<MODE>(a, outbuf);
 }
 
 }  // namespace kmsd
