@@ -35,7 +35,8 @@
 // Whole solves, block-Jacobi, rtol 1e-10, against the launch sequence:
 //   2,048 orbitals x 8 columns (cluster)    0.60 ms, 2.51 ms before
 //   6,912 x 13 (grid)                       0.95 ms, 3.19 ms
-//   32,000 x 32 (stream)                    4.5 ms,  8.0 ms
+//   32,000 x 32 (stream)                    4.6 ms,  8.2 ms
+//   55,296 x 16 (stream)                    4.5 ms,  9.4 ms
 // The grid form took 1.41 M cycles where the cluster form took 1.19 M on the
 // first, and 1.15 M against 1.07 M on 864 x 16; the stream form 2.74 M where the
 // grid form took 1.63 M on the second.
@@ -78,16 +79,19 @@ struct ResArgs {
 constexpr int kStateDoubles = 8, kStateInts = 4;
 constexpr int kAhead = 1;
 constexpr int kResThreads = 384, kStreamThreads = 512, kClusterCtas = 16;
-// 16-byte units from one S block in shared memory to the next: one more than
-// its 8, so that lanes on neighbouring blocks read from different banks.
-constexpr int kBlockUnits = 9;
+// 16-byte units from one S block in shared memory to the next: in the resident
+// forms one more than its 8, so that lanes on neighbouring blocks read from
+// different banks; in the stream form, whose warps read one block at a time, none
+// more, which lets shares of up to about 100 block rows of 16 blocks fit.
+constexpr int kResidentUnits = 9, kStreamUnits = 8;
 __host__ __device__ inline size_t up16(size_t x) { return (x + 15) / 16 * 16; }
 size_t state_bytes(int threads, int ncol, bool cluster) {
     return (size_t)(threads / 32) * ncol * 16 + (size_t)ncol * (16 + kStateDoubles * 8 + kStateInts * 4) +
            (cluster ? (size_t)2 * kClusterCtas * ncol * 16 : 0);
 }
-__host__ __device__ inline size_t slice_bytes(int own, int blocks, bool cplx, int pre_doubles, int halos) {
-    return (size_t)blocks * kBlockUnits * (cplx ? 32 : 16) + (size_t)own * pre_doubles * 8 +
+__host__ __device__ inline size_t slice_bytes(int own, int blocks, bool cplx, int pre_doubles, int halos,
+                                                      int units) {
+    return (size_t)blocks * units * (cplx ? 32 : 16) + (size_t)own * pre_doubles * 8 +
            up16(((size_t)blocks + 2 * (size_t)own + 1 + halos) * 4);
 }
 
@@ -229,6 +233,7 @@ __device__ __forceinline__ bool meet(unsigned *bar, unsigned &arrivals) {
 template <int lcw, bool CPLX, bool CL, bool RES>
 __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_resident_kernel(const ResArgs a) {
     constexpr int NT = RES ? kResThreads : kStreamThreads, NW = NT / 32, cw = 1 << lcw;
+    constexpr int kBlockUnits = RES ? kResidentUnits : kStreamUnits;
     extern __shared__ __align__(16) unsigned char sm[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ks = RES ? 1 << a.lks : 1, nch = RES ? 1 : a.nch, ncol = nch << lcw, b = a.b;
@@ -257,7 +262,7 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
     double *pre = reinterpret_cast<double *>(CPLX ? vim + (size_t)a.blocks * kBlockUnits : vim);
     int *sidx = reinterpret_cast<int *>(pre + (size_t)a.own * pre_d), *sptr = sidx + a.blocks, *sself = sptr + a.own + 1;
     int *shalo = sself + a.own;  // RES: the halo's block rows
-    double2 *stage = reinterpret_cast<double2 *>(slice + slice_bytes(a.own, a.blocks, CPLX, pre_d, RES ? a.halos : 0));
+    double2 *stage = reinterpret_cast<double2 *>(slice + slice_bytes(a.own, a.blocks, CPLX, pre_d, RES ? a.halos : 0, kBlockUnits));
     const int nhalo = RES ? a.halo_off[blockIdx.x + 1] - a.halo_off[blockIdx.x] : 0;
     {
         if constexpr (RES) {
@@ -1079,7 +1084,7 @@ int resident_plan(kmsd_metric_s *M, int64_t b, ResidentPlan *out) {
         if ((1 << full) < b || S->bsr_nb > (int64_t)ctas * (kResThreads >> full)) return KMSD_OK;
         if (int rc = halo_of(M, ctas, &h)) return rc;
         const bool cl = form == kFormCluster;
-        pl.smem = state_bytes(kResThreads, 1 << full, cl) + slice_bytes(h->own, h->blocks, cplx, pre_d, h->most) +
+        pl.smem = state_bytes(kResThreads, 1 << full, cl) + slice_bytes(h->own, h->blocks, cplx, pre_d, h->most, kResidentUnits) +
                   ((size_t)h->most << (full + 6));
         if (pl.smem > limit || h->own > kResThreads >> full) return KMSD_OK;
         pl.form = form;
@@ -1098,7 +1103,7 @@ int resident_plan(kmsd_metric_s *M, int64_t b, ResidentPlan *out) {
         kmsd_metric_s::Halo *h;
         if ((rc = halo_of(M, sms, &h))) return rc;
         pl.nch = (int)((b + (1 << full) - 1) >> full);
-        pl.smem = state_bytes(kStreamThreads, pl.nch << full, false) + slice_bytes(h->own, h->blocks, cplx, pre_d, 0);
+        pl.smem = state_bytes(kStreamThreads, pl.nch << full, false) + slice_bytes(h->own, h->blocks, cplx, pre_d, 0, kStreamUnits);
         if (pl.smem <= limit) {
             pl.form = kFormStream;
             pl.ctas = sms;
