@@ -389,8 +389,7 @@ void kmsd_batch_destroy(kmsd_batch bt);
  * declares m's segments to be its instances (kmsd_metric_set_segments).
  * kmsd_batch_moments then computes, per instance, mu_k = Re<S B, T_k(H~) B>
  * with T_k advanced by S^-1 H through one segmented PCG per step, in FP64,
- * with direct moments (KMSD_MOMENTS_DOUBLING is rejected) and without a
- * CUDA graph (the PCG loop stops on a polled device flag).  The handles stay
+ * with direct moments (KMSD_MOMENTS_DOUBLING is rejected).  The handles stay
  * owned by the caller and must outlive the batch's use of them. */
 int kmsd_batch_attach_metric(kmsd_batch bt, kmsd_csr h, kmsd_metric m, double rtol,
                              double atol, int maxiter);
@@ -403,6 +402,8 @@ int kmsd_batch_rows(kmsd_batch bt, int64_t *offsets);
  * of kmsd_engine_moments for each instance with its own window
  * (center[i], half[i]; host arrays).  b_in: the concatenated (sum N_i, b)
  * complex128 block (device); mu: (ninst, length, b) float64 (device).
+ * An orthogonal batch whose instances all fit a thread-block cluster (real
+ * rows of up to 8 entries, up to about 30,000 rows) is one launch.  Otherwise
  * use_graph = 1: the whole sequence of step and reduction kernels is
  * captured once into a CUDA graph per (buffers, shape) and replayed.
  * Synchronises the stream at the end. */

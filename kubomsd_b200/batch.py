@@ -2,10 +2,12 @@
 
 `B200Batch` wraps `kmsd_batch_*` (include/kmsd.h): many Hamiltonians of
 uneven size, such as disorder realisations, concatenated block-diagonally on
-the device (with their overlap matrices for a nonorthogonal basis).  One kernel per Chebyshev step covers all of
-them, with per-instance spectral windows and per-instance moment reductions.
-The whole step sequence is captured into a CUDA graph and replayed.  `tune()`
-picks the row-tile size by timing.  The moments of every instance equal those
+the device (with their overlap matrices for a nonorthogonal basis).  Small
+orthogonal instances take all steps in one launch of thread-block clusters.
+Otherwise one kernel per Chebyshev step covers all of them, with per-instance
+spectral windows and per-instance moment reductions; the whole step sequence is
+captured into a CUDA graph and replayed, and `tune()` picks its row-tile size by
+timing.  The moments of every instance equal those
 of a separate `B200Operators.moments` call on it.
 """
 from __future__ import annotations
@@ -21,8 +23,9 @@ from .native import DeviceCSR, _check, _ptr, _stream, _torch
 class B200Batch:
     """Moments of many independent instances in one call.
 
-    Orthogonal instances (`overlaps=None`): mixed or FP64, one step kernel per
-    Chebyshev step over all instances, replayed from a CUDA graph.
+    Orthogonal instances (`overlaps=None`): mixed or FP64, one launch of
+    clusters where every instance fits one, else one step kernel per Chebyshev
+    step over all instances, replayed from a CUDA graph.
     Nonorthogonal instances (`overlaps` = one S per instance, `blocks` = the
     block-Jacobi factors (a, b, L) of each instance in its own row numbering,
     or None for the diagonal preconditioner): direct moments
