@@ -475,6 +475,7 @@ int run_clusters(kmsd_batch_s *bt, const double2 *B, double *mu, int64_t b, int6
         else {
             if (cl.jobs.ensure(jobs.size() * sizeof(ClusterJob))) return KMSD_ECUDA;
             KMSD_CUDA(cudaMemcpy(cl.jobs.p, jobs.data(), jobs.size() * sizeof(ClusterJob), cudaMemcpyHostToDevice));
+            if (settle()) return KMSD_ECUDA;
         }
     }
     if (cl.plan.size == 0) return KMSD_OK;

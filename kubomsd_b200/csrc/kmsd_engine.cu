@@ -123,6 +123,7 @@ int Reducer::ensure(int grid, int ncol, int copies) {
     if (!ticket.p) {
         if (ticket.ensure(kTreeTickets * sizeof(Ticket))) return KMSD_ECUDA;
         KMSD_CUDA(cudaMemset(ticket.p, 0, kTreeTickets * sizeof(Ticket)));
+        if (settle()) return KMSD_ECUDA;
     }
     return KMSD_OK;
 }
@@ -151,7 +152,8 @@ int kmsd_csr_s::ensure_f32() {
         if (err != cudaSuccess) return err;
         for (int64_t i = 0; i < count; ++i) f[i] = (float)h[i];
         if ((err = cudaMalloc(d, f.size() * sizeof(float))) != cudaSuccess) return err;
-        return cudaMemcpy(*d, f.data(), count * sizeof(float), cudaMemcpyHostToDevice);
+        if ((err = cudaMemcpy(*d, f.data(), count * sizeof(float), cudaMemcpyHostToDevice)) != cudaSuccess) return err;
+        return cudaStreamSynchronize(cudaStreamLegacy);
     };
     cudaError_t err = convert(re64, nnz, &dre);
     if (err == cudaSuccess && complex_values) err = convert(im64, nnz, &dim);

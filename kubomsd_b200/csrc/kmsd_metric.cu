@@ -1025,6 +1025,7 @@ int kmsd_metric_s::ensure(int64_t b, int64_t state_cols) {
     if (!dcount.p) {
         if (dcount.ensure(sizeof(Counters))) return KMSD_ECUDA;
         KMSD_CUDA(cudaMemset(dcount.p, 0, sizeof(Counters)));
+        if (settle()) return KMSD_ECUDA;
     }
     if (!host_pinned.p) {
         void *h = nullptr;

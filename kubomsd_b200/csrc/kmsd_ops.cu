@@ -726,7 +726,7 @@ bool aligned_velocity(E *e, int x) {
     if (cudaMemcpy(d64, re.data(), m * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(d64 + m, im.data(), m * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(d32, re32.data(), m * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(d32 + m, im32.data(), m * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess)
+        cudaMemcpy(d32 + m, im32.data(), m * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess || settle())
         return false;
     // 2: purely imaginary (the lattice velocities), the real plane is not read
     e->vell_state[x] = std::all_of(re.begin(), re.end(), [](double v) { return v == 0.; }) ? 2 : 1;
@@ -816,7 +816,7 @@ bool imaginary_velocity(E *e, int x) {
     const std::vector<float> im32(im.begin(), im.end());
     if (e->vcsr64[x].ensure(im.size() * sizeof(double)) || e->vcsr32[x].ensure(im32.size() * sizeof(float))) return false;
     if (cudaMemcpy(e->vcsr64[x].p, im.data(), im.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(e->vcsr32[x].p, im32.data(), im32.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess)
+        cudaMemcpy(e->vcsr32[x].p, im32.data(), im32.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess || settle())
         return false;
     e->vcsr_state[x] = 1;
     return true;

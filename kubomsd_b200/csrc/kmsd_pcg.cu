@@ -1054,6 +1054,7 @@ int halo_of(kmsd_metric_s *M, int ctas, kmsd_metric_s::Halo **out) {
         *dst[i] = d;
         d += n[i];
     }
+    if (settle()) return KMSD_ECUDA;
     auto ins = M->halos.emplace(ctas, h);
     h.mem.p = nullptr;  // owned by the map entry now
     *out = &ins.first->second;
@@ -1118,6 +1119,7 @@ int resident_plan(kmsd_metric_s *M, int64_t b, ResidentPlan *out) {
     if (M->resident.bytes < bytes) {
         if (M->resident.ensure(bytes)) return KMSD_ECUDA;
         KMSD_CUDA(cudaMemset(M->resident.p, 0, bytes));
+        if (settle()) return KMSD_ECUDA;
     }
     if (M->ensure((int64_t)cols, b)) return KMSD_ECUDA;
     *out = pl;

@@ -83,3 +83,40 @@ def test_resident_solve_breakdown(cuda):
     metric, eng, cfg = _solve((D + 60. * (S - D)).tocsr(), [], B)  # indefinite, positive diagonal
     with pytest.raises(NumericalError, match="curvature breakdown"):
         metric.solve(B, cfg)
+
+
+@pytest.mark.parametrize("b", [8, 32])
+def test_first_solves_of_replicas_behind_large_copies(cuda, b):
+    """Block patterns and counters that a replica's first solve uploads are on
+    the device before its kernel runs, also while other streams keep the copy
+    engine busy; the solves are deterministic, so all agree bit for bit."""
+    import threading
+    import torch
+    from tests.gpu_util import engine
+    H, S, blocks = atom_model(400, 5)
+    metric, eng, _ = engine(H, S, blocks=blocks, rtol=RTOL)
+    rng = np.random.default_rng(b)
+    B = torch.from_numpy(rng.standard_normal((S.shape[0], b)) + 0j).cuda()
+    want = eng.h_action(B).cpu()
+    replicas = [eng.replica() for _ in range(4)]
+    host = torch.empty(1 << 28, dtype=torch.uint8).pin_memory()
+    dev = torch.empty(1 << 28, dtype=torch.uint8, device="cuda")
+    copies = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    got = [None] * len(replicas)
+
+    def first(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            got[i] = replicas[i].h_action(B).cpu()
+
+    with torch.cuda.stream(copies):
+        for _ in range(8):
+            dev.copy_(host, non_blocking=True)
+    threads = [threading.Thread(target=first, args=(i,)) for i in range(len(replicas))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for x in got:
+        assert torch.equal(x, want)
