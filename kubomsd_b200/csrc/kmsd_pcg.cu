@@ -614,7 +614,15 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
         for (int j = tid; j < ncol; j += NT) pend[j] = 0.;
     };
 
-    for (int k = 0; alive && !halt && k < a.maxiter; ++k) {
+    // A column leaves when its recurrence's residual meets the threshold; where the
+    // true residual, a few roundings away, then misses it, the column goes on from
+    // its true residual (`redo`) instead of failing the solve.
+    int k = 0, redos = 0;
+    bool redo = false;
+again:
+    for (; alive && !halt && k < a.maxiter; ++k) {
+        bool left = false;
+        if (!redo) {
         // ---- p = z + beta p, S p = S z + beta S p, <p, S p>
         for (int ch = 0; ch < nch; ++ch) {
             if constexpr (RES) fetch(a.z);
@@ -722,7 +730,7 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
             gather_sums(ch, acc, Sum{});
         }
         if (!(alive = reduce(Sum{}, std::true_type{}))) break;
-        bool cand = false, left = false;
+        bool cand = false;
         bool check = (k + 1) % a.interval == 0;
         for (int j = tid; j < b; j += NT) {
             const int act = active[j];
@@ -745,6 +753,7 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
             }
             halt = !__syncthreads_or(left);
             continue;
+        }
         }
         // ---- true residual t = q - S x; restart decision (native.cpp:379-402)
         __syncthreads();
@@ -780,7 +789,7 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
             int act = active[j], rst = 0;
             if (act) {
                 const double tn = sqrt(tot[j].x);
-                if (a.adaptive) {
+                if (a.adaptive && !redo) {
                     const double gap = sqrt(tot[j].y);
                     rst = tn > thr[j] && (gap > a.gap_ratio * fmax(tn, thr[j]) || rnorm[j] <= thr[j]);
                 } else {
@@ -833,6 +842,7 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
             rz[j] = now;
             left |= active[j] != 0;
         }
+        redo = false;
         halt = !__syncthreads_or(left);
     }
 
@@ -882,6 +892,20 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
             gather_sums(ch, acc, Sum{});
         }
         alive = alive && reduce(Sum{}, std::false_type{});
+    }
+    if (alive && !broken && !nonfinite && k < a.maxiter && redos < 4) {
+        bool more = false;
+        for (int j = tid; j < b; j += NT) {
+            active[j] = rnorm[j] > thr[j] && !brk[j];
+            more |= active[j] != 0;
+        }
+        if (__syncthreads_or(more)) {
+            ++redos;
+            redo = true;
+            halt = 0;
+            --k;
+            goto again;
+        }
     }
     if (blockIdx.x != 0) return;
     // the packets of a solve that gave up may be some numbers ahead
