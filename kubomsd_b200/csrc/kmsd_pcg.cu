@@ -124,16 +124,17 @@ struct Patience {
 };
 // A double as a packet whose 8-byte halves each carry half of it and the
 // sequence number: a reader that finds the number in both has the value, so a
-// reduction takes one trip through L2 instead of a counter's and the data's.
+// reduction takes one trip through L2 instead of a counter's and the data's.  Each
+// half is one 64-bit element of the vector access, so a half is never torn.
 __device__ __forceinline__ void packet_store(uint4 *p, double v, unsigned seq) {
-    asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"((unsigned)__double2loint(v)), "r"(seq),
-                 "r"((unsigned)__double2hiint(v)), "r"(seq)
-                 : "memory");
+    const unsigned long long lo = (unsigned long long)seq << 32 | (unsigned)__double2loint(v),
+                             hi = (unsigned long long)seq << 32 | (unsigned)__double2hiint(v);
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(lo), "l"(hi) : "memory");
 }
 __device__ __forceinline__ uint4 packet_load(const uint4 *p) {
-    uint4 v;
-    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
-    return v;
+    unsigned long long lo, hi;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
+    return make_uint4((unsigned)lo, (unsigned)(lo >> 32), (unsigned)hi, (unsigned)(hi >> 32));
 }
 __device__ __forceinline__ double packet_value(const uint4 &v) { return __hiloint2double((int)v.z, (int)v.x); }
 __device__ __forceinline__ void copy16(void *smem, const void *global) {
@@ -205,6 +206,19 @@ __device__ __noinline__ bool totals(const uint4 *in, double2 *tot, int ncol, uns
     return late;
 }
 
+// The two halves of a meeting of a cooperative launch, at a counter: what the CTA
+// wrote before (its threads synchronised) is visible to a thread that has waited for
+// all arrivals, and to its CTA once that has synchronised.
+__device__ __forceinline__ void arrive(unsigned *bar) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+}
+// True when the wait ran out.
+__device__ __forceinline__ bool wait_for(unsigned *bar, unsigned arrivals) {
+    Patience wait;
+    while ((int)(load_acquire(bar) - arrivals) < 0)
+        if (wait.out(bar)) return true;
+    return false;
+}
 // All CTAs of the solve have arrived, and their writes are visible.  CL: the
 // solve is one thread-block cluster and meets at the hardware barrier; else the
 // launch is cooperative and meets at a counter, with a bounded wait.
@@ -218,10 +232,8 @@ __device__ __forceinline__ bool meet(unsigned *bar, unsigned &arrivals) {
         arrivals += gridDim.x;
         bool late = false;
         if (threadIdx.x == 0) {
-            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-            Patience wait;
-            while ((int)(load_acquire(bar) - arrivals) < 0)
-                if ((late = wait.out(bar))) break;
+            arrive(bar);
+            late = wait_for(bar, arrivals);
         }
         return !__syncthreads_or(late);
     }
@@ -305,9 +317,10 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
         if (lane < cw) red[warp * ncol + (ch << lcw) + lane] = v;
     };
     // Column sums over all CTAs into tot (in every CTA), in a fixed order:
-    // lanes, warps, CTAs.  Max: the largest value instead.  PUBLISH: writes of
-    // this CTA before the call are visible to the others after it.
-    auto reduce = [&](auto maximum, auto publish) -> bool {
+    // lanes, warps, CTAs.  Max: the largest value instead.  It is a meeting too:
+    // what the CTAs read and wrote before it comes before what any of them reads
+    // and writes after it.
+    auto reduce = [&](auto maximum) -> bool {
         constexpr bool MX = decltype(maximum)::value;
         auto join = [](double2 &s, double2 q) {
             s.x = MX ? fmax(s.x, q.x) : s.x + q.x;
@@ -340,7 +353,13 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
             __syncthreads();
             return true;
         } else {
-            constexpr bool PUBLISH = decltype(publish)::value;
+            // The totals order nothing but themselves: the CTA that sums a column
+            // puts no fence between its reads and its store.  The CTAs meet at the
+            // counter besides, in the last warp and in the shadow of the sums, which
+            // take a trip more.  (With fences around the packets and in
+            // column_total() a solve of 6,912 x 13 took 1.00 ms, with this 0.88.)
+            arrivals += gridDim.x;
+            if (tid == NT - 1) arrive(a.bar);
             uint4 *all = a.packets + (size_t)buf * ncol * (gridDim.x + 1) * 2, *sums = all + (size_t)ncol * gridDim.x * 2;
             buf ^= 1;
             ++seq;
@@ -348,7 +367,6 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
                 double2 s = red[j];
 #pragma unroll 4
                 for (int w = 1; w < NW; ++w) join(s, red[w * ncol + j]);
-                if (PUBLISH) __threadfence();
                 uint4 *mine = all + ((size_t)j * gridDim.x + blockIdx.x) * 2;
                 packet_store(mine, s.x, seq);
                 packet_store(mine + 1, s.y, seq);
@@ -358,7 +376,7 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
             for (int j = blockIdx.x + warp * gridDim.x; j < ncol; j += NW * gridDim.x)
                 late |= column_total<MX>(all + (size_t)j * gridDim.x * 2, sums + 2 * j, seq, a.bar);
             late |= totals(sums, tot, ncol, seq, a.bar);
-            if (PUBLISH) __threadfence();
+            if (tid == NT - 1) late |= wait_for(a.bar, arrivals);
             return !__syncthreads_or(late);
         }
     };
@@ -530,7 +548,7 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
         });
         gather_sums(ch, m, Max{});
     }
-    alive = reduce(Max{}, std::false_type{});
+    alive = reduce(Max{});
     bool nan_in = false;
     for (int j = tid; j < ncol; j += NT) {
         safe[j] = tot[j].x == 0. ? 1. : tot[j].x;
@@ -570,7 +588,7 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
         });
         gather_sums(ch, acc, Sum{});
     }
-    alive = alive && reduce(Sum{}, std::true_type{});
+    alive = alive && reduce(Sum{});
     bool todo = false;
     for (int j = tid; j < ncol; j += NT) {
         bn[j] = sqrt(tot[j].x);
@@ -676,7 +694,7 @@ again:
             });
             gather_sums(ch, acc, Sum{});
         }
-        if (!(alive = reduce(Sum{}, std::false_type{}))) break;
+        if (!(alive = reduce(Sum{}))) break;
         bool bad = false;
         for (int j = tid; j < b; j += NT) {
             const double cr = tot[j].x, ci = tot[j].y;
@@ -729,7 +747,7 @@ again:
             });
             gather_sums(ch, acc, Sum{});
         }
-        if (!(alive = reduce(Sum{}, std::true_type{}))) break;
+        if (!(alive = reduce(Sum{}))) break;
         bool cand = false;
         bool check = (k + 1) % a.interval == 0;
         for (int j = tid; j < b; j += NT) {
@@ -783,7 +801,7 @@ again:
             });
             gather_sums(ch, acc, Sum{});
         }
-        if (!(alive = reduce(Sum{}, std::false_type{}))) break;
+        if (!(alive = reduce(Sum{}))) break;
         int nrs = 0;
         for (int j = tid; j < b; j += NT) {
             int act = active[j], rst = 0;
@@ -835,7 +853,7 @@ again:
             });
             gather_sums(ch, acc, Sum{});
         }
-        if (!(alive = reduce(Sum{}, std::true_type{}))) break;
+        if (!(alive = reduce(Sum{}))) break;
         for (int j = tid; j < b; j += NT) {
             const double old = rz[j], now = tot[j].y;
             beta[j] = active[j] ? now / (old != 0. ? old : 1.) : 0.;
@@ -871,7 +889,7 @@ again:
             });
             gather_sums(ch, acc, Sum{});
         }
-        alive = reduce(Sum{}, std::false_type{});
+        alive = reduce(Sum{});
         for (int j = tid; j < b; j += NT) rnorm[j] = sqrt(tot[j].x);
         for (int ch = 0; ch < nch; ++ch) {
             double2 acc = make_double2(0., 0.);
@@ -891,7 +909,7 @@ again:
             });
             gather_sums(ch, acc, Sum{});
         }
-        alive = alive && reduce(Sum{}, std::false_type{});
+        alive = alive && reduce(Sum{});
     }
     if (alive && !broken && !nonfinite && k < a.maxiter && redos < 4) {
         bool more = false;
