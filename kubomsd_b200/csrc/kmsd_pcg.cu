@@ -298,9 +298,14 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
             else pre[i] = reinterpret_cast<const double *>(a.minv + 16 * I0)[i];
         }
     }
-    const unsigned base = CL ? 0u : *(volatile unsigned *)(a.bar + 2);
-    if constexpr (CL) cluster_meet();  // every CTA of the cluster is running before its boxes are written
-    else __syncthreads();
+    unsigned base = 0;
+    bool gone = false;  // the others gave up before this CTA began
+    if constexpr (CL) {
+        cluster_meet();  // every CTA of the cluster is running before its boxes are written
+    } else {
+        base = load_acquire(a.bar + 2);
+        gone = __syncthreads_or(load_acquire(a.bar + 1));
+    }
 
     unsigned arrivals = 0, seq = base;
     int buf = 0;
@@ -548,7 +553,7 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
         });
         gather_sums(ch, m, Max{});
     }
-    alive = reduce(Max{});
+    alive = !gone && reduce(Max{});
     bool nan_in = false;
     for (int j = tid; j < ncol; j += NT) {
         safe[j] = tot[j].x == 0. ? 1. : tot[j].x;
@@ -926,8 +931,13 @@ again:
         }
     }
     if (blockIdx.x != 0) return;
-    // the packets of a solve that gave up may be some numbers ahead
-    if (!CL && tid == 0) a.bar[2] = seq + (alive ? 0u : 1024u);
+    // The packets of a solve that gave up may be some numbers ahead.  A CTA that
+    // begins after this and reads the new base finds bar[1] set and puts out none,
+    // which the next solve would take for its own.
+    if (!CL && tid == 0) {
+        __threadfence();
+        a.bar[2] = seq + (alive ? 0u : 1024u);
+    }
     if (!alive) {
         if (tid == 0) atomicOr(a.status + 3, 1);
         return;
