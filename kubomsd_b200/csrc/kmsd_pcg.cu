@@ -896,6 +896,23 @@ again:
         }
         alive = reduce(Sum{});
         for (int j = tid; j < b; j += NT) rnorm[j] = sqrt(tot[j].x);
+    }
+    if (alive && !broken && !nonfinite && k < a.maxiter && redos < 4) {
+        bool more = false;
+        for (int j = tid; j < b; j += NT) {
+            active[j] = rnorm[j] > thr[j] && !brk[j];
+            more |= active[j] != 0;
+        }
+        if (__syncthreads_or(more)) {
+            ++redos;
+            redo = true;
+            halt = 0;
+            --k;
+            goto again;
+        }
+    }
+    // (only now: Y may be B, which the continuation reads again)
+    if (alive) {
         for (int ch = 0; ch < nch; ++ch) {
             double2 acc = make_double2(0., 0.);
             rows(ch, [&](int li, bool on, int u) {
@@ -914,21 +931,7 @@ again:
             });
             gather_sums(ch, acc, Sum{});
         }
-        alive = alive && reduce(Sum{});
-    }
-    if (alive && !broken && !nonfinite && k < a.maxiter && redos < 4) {
-        bool more = false;
-        for (int j = tid; j < b; j += NT) {
-            active[j] = rnorm[j] > thr[j] && !brk[j];
-            more |= active[j] != 0;
-        }
-        if (__syncthreads_or(more)) {
-            ++redos;
-            redo = true;
-            halt = 0;
-            --k;
-            goto again;
-        }
+        alive = reduce(Sum{});
     }
     if (blockIdx.x != 0) return;
     // The packets of a solve that gave up may be some numbers ahead.  A CTA that
