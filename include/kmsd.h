@@ -80,7 +80,7 @@ typedef struct {
     int64_t true_residual_refreshes;
     int64_t true_residual_checks;
     int64_t residual_restarts;
-    int64_t refinement_steps;
+    int64_t refinement_steps; /* solves that went on from their true residual after an acceptance missed by roundings */
 } kmsd_metric_stats;
 
 /* ---- library ---------------------------------------------------------- */

@@ -1830,7 +1830,7 @@ int kmsd_metric_stats_get(kmsd_metric m, kmsd_metric_stats *out) {
     out->true_residual_refreshes = c.v[0];
     out->true_residual_checks = c.v[1];
     out->residual_restarts = c.v[2];
-    out->refinement_steps = 0;
+    out->refinement_steps = c.redos;
     return KMSD_OK;
 }
 

@@ -31,10 +31,12 @@ inline ColPtr col_ptr(void *base, int64_t b) {
     c.flags = ip + (size_t)kInts * b;
     return c;
 }
-// device counters: [0] refreshes [1] checks [2] restarts [3] iterations sum; [4] max relative (double bits)
+// device counters: [0] refreshes [1] checks [2] restarts [3] iterations sum; max
+// relative residual; continuations of one-launch solves
 struct Counters {
     long long v[4];
     double max_rel;
+    long long redos;
 };
 
 struct Pre {

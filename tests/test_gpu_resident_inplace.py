@@ -41,3 +41,31 @@ def test_solution_over_its_right_hand_side(cuda, b):
         assert _solve(torch, metric, over, over, 1e-14) == rc  # (a column may miss for good, then in both)
         if rc == 0:
             assert torch.equal(over, apart)
+
+
+@pytest.mark.parametrize("b", [8, 32, 64])
+def test_columns_that_just_miss_go_on(cuda, b):
+    """A column above its threshold by at most 1/1024 goes on and converges, and the
+    solve is counted (kmsd_metric_stats.refinement_steps); one that is further off
+    fails the solve with its residual."""
+    from kubomsd_b200.errors import NumericalError
+    torch = cuda
+    rtol = 1e-14
+    metric, S = _diamond()
+    cfg = metric._create[2]
+    cfg.metric_rtol = rtol
+    A = torch.sparse_csr_tensor(torch.from_numpy(S.indptr.astype(np.int64)), torch.from_numpy(S.indices.astype(np.int64)),
+                                torch.from_numpy(S.data.astype(complex)), size=S.shape).cuda()
+    g = torch.Generator(device="cuda").manual_seed(b)
+    for _ in range(8000 // b):
+        B = torch.randn((S.shape[0], b), dtype=torch.complex128, device="cuda", generator=g)
+        try:
+            x, report = metric.solve(B, cfg)
+        except NumericalError as exc:
+            rel = np.array(exc.diagnostics["relative_residual"])
+            assert rel[~np.array(exc.diagnostics["converged"])].min() > rtol * (1 + 1 / 1024) * (1 - 1e-9)
+            continue
+        assert report.converged.all() and report.relative_residual.max() <= rtol * (1 + 1e-9)
+        # formed once more, with roundings of about a hundredth of the threshold at most
+        assert float(((B - A @ x).norm(dim=0) / B.norm(dim=0)).max()) <= 1.1 * rtol
+    assert metric.stats().refinement_steps > 0
