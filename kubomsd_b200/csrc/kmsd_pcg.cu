@@ -643,7 +643,8 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
 
     int k = 0, redos = 0;
     while (true) {
-        for (; alive && !halt && k < a.maxiter; ++k) {
+        bool accept = true;  // the next true residual decides the solve
+        while (alive && !halt && !broken && k < a.maxiter) {
             // ---- p = z + beta p, S p = S z + beta S p, <p, S p>
             for (int ch = 0; ch < nch; ++ch) {
                 if constexpr (RES) fetch(a.z);
@@ -761,117 +762,29 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
                 cand |= act && rnorm[j] <= thr[j];
             }
             if (a.adaptive) check = __syncthreads_or(cand) || check;
-            if (!check) {
-                for (int j = tid; j < b; j += NT) {
-                    int act = active[j];
-                    if (!a.adaptive) act = act && rnorm[j] > thr[j];
-                    active[j] = act;
-                    restart[j] = 0;
-                    const double old = rz[j], now = tot[j].y;
-                    beta[j] = act ? now / (old != 0. ? old : 1.) : 0.;
-                    rz[j] = now;
-                    left |= act != 0;
-                }
-                halt = !__syncthreads_or(left);
-                continue;
+            ++k;
+            if (check) {
+                accept = false;
+                break;
             }
-            // ---- true residual t = q - S x; restart decision (native.cpp:379-402)
-            __syncthreads();
-            flush();
-            if (!(alive = meet<CL>(a.bar, arrivals))) break;
-            for (int ch = 0; ch < nch; ++ch) {
-                if constexpr (RES) fetch(a.y);
-                double2 acc = make_double2(0., 0.);
-                rows(ch, [&](int li, bool on, int u) {
-                    double2 w[4];
-                    product(a.y, ch, li, on, w);
-                    if (!on) return;
-                    const double sf = safe[u];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const size_t o = at(ch, li, i);
-                        const double2 v = input(li, i, u);
-                        const double2 t = make_double2(v.x / sf - w[i].x, v.y / sf - w[i].y);
-                        const double2 rv = RES ? rs[i] : a.r[o];
-                        if (first) {
-                            a.t[o] = t;
-                            acc.x += t.x * t.x + t.y * t.y;
-                            const double dx = t.x - rv.x, dy = t.y - rv.y;
-                            acc.y += dx * dx + dy * dy;
-                        }
-                    }
-                });
-                gather_sums(ch, acc, Sum{});
-            }
-            if (!(alive = reduce(Sum{}))) break;
-            int nrs = 0;
             for (int j = tid; j < b; j += NT) {
-                int act = active[j], rst = 0;
-                if (act) {
-                    const double tn = sqrt(tot[j].x);
-                    if (a.adaptive) {
-                        const double gap = sqrt(tot[j].y);
-                        rst = tn > thr[j] && (gap > a.gap_ratio * fmax(tn, thr[j]) || rnorm[j] <= thr[j]);
-                    } else {
-                        rst = 1;
-                    }
-                    act = tn > thr[j];
-                }
+                int act = active[j];
+                if (!a.adaptive) act = act && rnorm[j] > thr[j];
                 active[j] = act;
-                restart[j] = rst;
-                nrs += rst;
-            }
-            ++checks;
-            restarts += __syncthreads_count(nrs != 0);
-            // ---- r <- t on restarted columns, z = M^-1 r
-            for (int ch = 0; ch < nch; ++ch) {
-                double2 acc = make_double2(0., 0.);
-                rows(ch, [&](int li, bool on, int u) {
-                    if (!on) return;
-                    const bool rst = restart[u];
-                    double2 rr[4], zz[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const size_t o = at(ch, li, i);
-                        if constexpr (RES) {
-                            if (rst) rs[i] = __ldcg(a.t + o);
-                            rr[i] = rs[i];
-                        } else {
-                            rr[i] = rst ? a.t[o] : a.r[o];
-                        }
-                    }
-                    precondition(li, rr, zz);
-                    if (first) {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const size_t o = at(ch, li, i);
-                            a.z[o] = zz[i];
-                            if constexpr (!RES) {
-                                if (rst) a.r[o] = rr[i];
-                            }
-                            acc.y += rr[i].x * zz[i].x + rr[i].y * zz[i].y;
-                        }
-                    }
-                });
-                gather_sums(ch, acc, Sum{});
-            }
-            if (!(alive = reduce(Sum{}))) break;
-            for (int j = tid; j < b; j += NT) {
+                restart[j] = 0;
                 const double old = rz[j], now = tot[j].y;
-                beta[j] = active[j] ? now / (old != 0. ? old : 1.) : 0.;
+                beta[j] = act ? now / (old != 0. ? old : 1.) : 0.;
                 rz[j] = now;
-                left |= active[j] != 0;
+                left |= act != 0;
             }
             halt = !__syncthreads_or(left);
         }
-
-        // ---- acceptance: t = q - S x (native.cpp:413-423)
-        if (alive) {
-            __syncthreads();
-            flush();
-            alive = meet<CL>(a.bar, arrivals);
-        }
         if (!alive) break;
+        // ---- true residual t = q - S x: restart decision (native.cpp:379-402) or
+        // acceptance (native.cpp:413-423)
+        __syncthreads();
+        flush();
+        if (!(alive = meet<CL>(a.bar, arrivals))) break;
         for (int ch = 0; ch < nch; ++ch) {
             if constexpr (RES) fetch(a.y);
             double2 acc = make_double2(0., 0.);
@@ -882,49 +795,81 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
                 const double sf = safe[u];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
+                    const size_t o = at(ch, li, i);
                     const double2 v = input(li, i, u);
                     const double2 t = make_double2(v.x / sf - w[i].x, v.y / sf - w[i].y);
-                    if constexpr (RES) rs[i] = t;
+                    const double2 rv = RES ? rs[i] : a.r[o];
                     if (first) {
-                        if constexpr (!RES) a.r[at(ch, li, i)] = t;
+                        a.t[o] = t;
                         acc.x += t.x * t.x + t.y * t.y;
+                        const double dx = t.x - rv.x, dy = t.y - rv.y;
+                        acc.y += dx * dx + dy * dy;
                     }
                 }
             });
             gather_sums(ch, acc, Sum{});
         }
         if (!(alive = reduce(Sum{}))) break;
-        // Under the fixed policy a column leaves when the residual of its recurrence
-        // meets the threshold.  The true one is some roundings away, 1e-7 of the
-        // threshold at a tolerance of 1e-10 (5e-4 at 1e-13), and misses it in about one
-        // of 10^7 columns.  Such a column goes on from its true residual, which r holds
-        // by now; one that is further off than roundings explain fails.
         bool more = false;
         for (int j = tid; j < b; j += NT) {
-            rnorm[j] = sqrt(tot[j].x);
-            active[j] = !broken && !nonfinite && k < a.maxiter && redos < kMostRedos && rnorm[j] > thr[j] &&
-                        rnorm[j] <= kRedoWithin * thr[j];
-            restart[j] = 1;
-            more |= active[j] != 0;
+            const double tn = sqrt(tot[j].x);
+            int act = active[j], rst = 0;
+            if (accept) {
+                // Under the fixed policy a column leaves when the residual of its
+                // recurrence meets the threshold.  The true one is some roundings
+                // away, 1e-7 of the threshold at a tolerance of 1e-10 (5e-4 at
+                // 1e-13), and misses it in about one of 10^7 columns.  Such a column
+                // goes on from its true residual; one that is further off than
+                // roundings explain fails.
+                rnorm[j] = tn;
+                act = rst = !broken && !nonfinite && k < a.maxiter && redos < kMostRedos && tn > thr[j] &&
+                            tn <= kRedoWithin * thr[j];
+            } else if (act) {
+                if (a.adaptive) {
+                    const double gap = sqrt(tot[j].y);
+                    rst = tn > thr[j] && (gap > a.gap_ratio * fmax(tn, thr[j]) || rnorm[j] <= thr[j]);
+                } else {
+                    rst = 1;
+                }
+                act = tn > thr[j];
+            }
+            active[j] = act;
+            restart[j] = rst;
+            more |= rst != 0;
         }
-        if (!__syncthreads_or(more)) break;
-        ++redos;
-        halt = 0;
+        if (accept) {
+            if (!__syncthreads_or(more)) break;
+            ++redos;
+        } else {
+            ++checks;
+            restarts += __syncthreads_count(more);
+        }
+        // ---- r <- t on restarted columns, z = M^-1 r
         for (int ch = 0; ch < nch; ++ch) {
             double2 acc = make_double2(0., 0.);
             rows(ch, [&](int li, bool on, int u) {
                 if (!on) return;
+                const bool rst = restart[u];
                 double2 rr[4], zz[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    if constexpr (RES) rr[i] = rs[i];
-                    else rr[i] = a.r[at(ch, li, i)];
+                    const size_t o = at(ch, li, i);
+                    if constexpr (RES) {
+                        if (rst) rs[i] = __ldcg(a.t + o);
+                        rr[i] = rs[i];
+                    } else {
+                        rr[i] = rst ? a.t[o] : a.r[o];
+                    }
                 }
                 precondition(li, rr, zz);
                 if (first) {
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
-                        a.z[at(ch, li, i)] = zz[i];
+                        const size_t o = at(ch, li, i);
+                        a.z[o] = zz[i];
+                        if constexpr (!RES) {
+                            if (rst) a.r[o] = rr[i];
+                        }
                         acc.y += rr[i].x * zz[i].x + rr[i].y * zz[i].y;
                     }
                 }
@@ -932,8 +877,14 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
             gather_sums(ch, acc, Sum{});
         }
         if (!(alive = reduce(Sum{}))) break;
-        for (int j = tid; j < b; j += NT) rz[j] = tot[j].y;
-        __syncthreads();
+        bool left = false;
+        for (int j = tid; j < b; j += NT) {
+            const double old = rz[j], now = tot[j].y;
+            beta[j] = active[j] ? now / (old != 0. ? old : 1.) : 0.;
+            rz[j] = now;
+            left |= active[j] != 0;
+        }
+        halt = !__syncthreads_or(left);
     }
 
     // ---- Y = x safe, with the representability checks (native.cpp:424-444)
