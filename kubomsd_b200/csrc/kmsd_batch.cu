@@ -264,6 +264,7 @@ int build_tiles(kmsd_batch_s *bt, int64_t tile_rows) {
     KMSD_CUDA(cudaMemcpy(bt->tiles.r1, r1.data(), nt * sizeof(int64_t), cudaMemcpyHostToDevice));
     KMSD_CUDA(cudaMemcpy(bt->tiles.seg, seg.data(), nt * sizeof(int), cudaMemcpyHostToDevice));
     KMSD_CUDA(cudaMemcpy(bt->tiles.seg_tile0, first.data(), (bt->ninst + 1) * sizeof(int), cudaMemcpyHostToDevice));
+    if (settle()) return KMSD_ECUDA;
     bt->tiles.ntiles = nt;
     bt->tiles.tile_rows = tile_rows;
     for (auto &kv : bt->graphs) cudaGraphExecDestroy(kv.second);

@@ -464,6 +464,7 @@ int kmsd_csr_create(int64_t n, const int64_t *indptr, const int64_t *indices, co
             }
         }
     }
+    if (!rc && settle()) rc = KMSD_ECUDA;
     if (rc) {
         kmsd_csr_destroy(A);
         return rc;

@@ -25,11 +25,14 @@ int cuda_fail(cudaError_t e, const char *what);
         if (e_ != cudaSuccess) return cuda_fail(e_, #call);  \
     } while (0)
 
-// Waits for first-use copies and clears: a cudaMemcpy from pageable memory may
+// Waits for uploads and clears: a cudaMemcpy from pageable memory may
 // return with its last part still under way and a cudaMemset is asynchronous,
 // both on the legacy stream, for which non-blocking streams do not wait.  True on
 // an error.
-inline bool settle() { return cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess; }
+inline bool settle() {
+    const cudaError_t e = cudaStreamSynchronize(cudaStreamLegacy);
+    return e != cudaSuccess && cuda_fail(e, "an upload");
+}
 
 // Grow-only device buffer.
 struct DevBuf {

@@ -1085,6 +1085,7 @@ int kmsd_metric_s::seg_plan(int gpc, SegPlan **out) {
     KMSD_CUDA(cudaMemcpy(base + o_cta0, cta0.data(), (ns + 1) * 4, cudaMemcpyHostToDevice));
     KMSD_CUDA(cudaMemcpy(base + o_tk0, tk0.data(), (ns + 1) * 4, cudaMemcpyHostToDevice));
     KMSD_CUDA(cudaMemcpy(base + o_l2, l2.data(), ns * 4, cudaMemcpyHostToDevice));
+    if (settle()) return KMSD_ECUDA;
     pl.row0 = reinterpret_cast<int64_t *>(base + o_row);
     pl.blk0 = reinterpret_cast<int64_t *>(base + o_blk);
     pl.cta_seg = reinterpret_cast<int *>(base + o_cseg);
@@ -1690,6 +1691,7 @@ int kmsd_metric_create(kmsd_csr s, const double *diag, int64_t nblocks, const in
         if (!rc) rc = up((void **)&M->foff, offs.data(), offs.size() * sizeof(int64_t));
         if (!rc) rc = up((void **)&M->factors, fac.data(), fac.size() * sizeof(double2));
     }
+    if (!rc && settle()) rc = KMSD_ECUDA;
     if (rc) {
         kmsd_metric_destroy(M);
         return rc;
