@@ -166,6 +166,7 @@ __global__ void __launch_bounds__(kMaxCompute<T> + 32, 1) cluster_moments_kernel
                 const int kk = i / nv, v = i - kk * nv;
                 out[((size_t)(first + kk) * size + rank) * nv + v] = hist[i];
             }
+            __syncwarp();  // the next sums go over this history; no meeting orders the lanes of this warp
         }
     };
     // The sums of CG columns from c on, over the warp, for step `sum`.
