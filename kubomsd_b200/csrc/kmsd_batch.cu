@@ -466,19 +466,26 @@ int run_clusters(kmsd_batch_s *bt, const double2 *B, double *mu, int64_t b, int6
                  bool *done) {
     *done = false;
     if (bt->width == 0 || length < 2) return KMSD_OK;
-    auto &cl = bt->clusters[{b, doubling}];
-    if (!cl.jobs.p && cl.plan.groups == 0) {
+    auto found = bt->clusters.find({b, doubling});
+    if (found == bt->clusters.end()) {
         std::vector<int64_t> rows(bt->ninst);
         for (int64_t i = 0; i < bt->ninst; ++i) rows[i] = bt->row_off[i + 1] - bt->row_off[i];
+        kmsd_batch_s::Clusters made;
         std::vector<ClusterJob> jobs;
-        if (int rc = cluster_batch_plan<T>(rows, bt->width, b, doubling, &cl.plan, &jobs)) return rc;
-        if (cl.plan.size == 0) cl.plan.groups = -1;  // decided: does not apply
-        else {
-            if (cl.jobs.ensure(jobs.size() * sizeof(ClusterJob))) return KMSD_ECUDA;
-            KMSD_CUDA(cudaMemcpy(cl.jobs.p, jobs.data(), jobs.size() * sizeof(ClusterJob), cudaMemcpyHostToDevice));
-            if (settle()) return KMSD_ECUDA;
+        if (int rc = cluster_batch_plan<T>(rows, bt->width, b, doubling, &made.plan, &jobs)) return rc;
+        if (made.plan.size != 0) {
+            const size_t bytes = jobs.size() * sizeof(ClusterJob);
+            if (made.jobs.ensure(bytes)) return KMSD_ECUDA;
+            const cudaError_t e = cudaMemcpy(made.jobs.p, jobs.data(), bytes, cudaMemcpyHostToDevice);
+            if (e != cudaSuccess || settle()) {
+                made.jobs.release();
+                return e != cudaSuccess ? cuda_fail(e, "cudaMemcpy (cluster jobs)") : KMSD_ECUDA;
+            }
         }
+        // last: an entry is complete, with its table on the device (size 0: does not apply)
+        found = bt->clusters.emplace(std::make_pair(b, doubling), made).first;
     }
+    const auto &cl = found->second;
     if (cl.plan.size == 0) return KMSD_OK;
     std::vector<ClusterSystem> sys(bt->ninst);
     for (int64_t i = 0; i < bt->ninst; ++i)
