@@ -92,6 +92,13 @@ def _dptr(a: np.ndarray):
     return a.ctypes.data_as(C.POINTER(C.c_double))
 
 
+def _plain(t):
+    """`t` with its values in memory as they read: contiguous, and neither lazily
+    conjugated nor lazily negated (`contiguous()` and `to()` keep both marks, and the
+    library reads memory)."""
+    return t.resolve_conj().resolve_neg().contiguous()
+
+
 def _finite(torch, t):
     """Whether every value of a contiguous complex128 CUDA tensor is finite: one
     pass over it (torch's isfinite().all() makes five: on 4,194,304 x 64 values
@@ -109,7 +116,7 @@ def as_device(B, n=None, validate=True):
     if isinstance(B, torch.Tensor):
         if B.ndim != 2 or B.shape[0] < 1 or B.shape[1] < 1:
             raise ValueError("expected nonempty finite (N,batch) array")
-        t = B.to(device="cuda", dtype=torch.complex128).contiguous()
+        t = _plain(B.to(device="cuda", dtype=torch.complex128))
         if validate and not _finite(torch, t):
             raise ValueError("expected finite (N,batch) array")
         host = False
@@ -632,7 +639,7 @@ class B200Operators:
         t, _ = as_device(B, self.n)
         b = t.shape[1]
         cov = cov if isinstance(cov, torch.Tensor) else torch.from_numpy(np.ascontiguousarray(cov, np.complex128))
-        cov = cov.to(t.device, torch.complex128)
+        cov = _plain(cov.to(t.device, torch.complex128))
         if length < 1:
             raise ValueError("Chebyshev chain must be nonempty")
         if cov.ndim != 3 or cov.shape[0] != self.n or cov.shape[2] != b:
