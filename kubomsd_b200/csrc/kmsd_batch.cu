@@ -626,10 +626,6 @@ int batch_call(kmsd_batch_s *bt, const void *b_in, double *mu, int64_t b, int64_
         auto it = bt->graphs.find(key);
         if (it == bt->graphs.end()) {
             if (!bt->cap) KMSD_CUDA(cudaStreamCreateWithFlags(&bt->cap, cudaStreamNonBlocking));
-            // the SpMMs size this thread's reduction buffers on first use:
-            // run them once outside the capture
-            if ((rc = spmm64(bt->gm->S, B, bt->t1.as<double2>(), b, s))) return rc;
-            if ((rc = spmm64(bt->gh, B, bt->t1.as<double2>(), b, s))) return rc;
             KMSD_CUDA(cudaStreamSynchronize(s));
             cudaGraph_t g = nullptr;
             int64_t recorded = 0;

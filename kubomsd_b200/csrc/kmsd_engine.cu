@@ -119,7 +119,7 @@ size_t reduce_smem(const RowMap &mp, int C) {
     return std::max(a, b) * sizeof(double2);
 }
 int Reducer::ensure(int grid, int ncol, int copies) {
-    if (partial.ensure((size_t)tree_rows(grid) * ncol * copies * sizeof(double2) + 64)) return KMSD_ECUDA;
+    if (partial.ensure(bytes(grid, ncol * copies))) return KMSD_ECUDA;
     if (!ticket.p) {
         if (ticket.ensure(kTreeTickets * sizeof(Ticket))) return KMSD_ECUDA;
         KMSD_CUDA(cudaMemset(ticket.p, 0, kTreeTickets * sizeof(Ticket)));
@@ -170,9 +170,71 @@ int kmsd_csr_s::ensure_f32() {
 }
 
 namespace {
+// Scratch of the column sums that belong to no engine or metric, one per device and
+// stream of a thread: launches that share a ticket have to run one after another,
+// which only those of one stream do.  Given back when the thread ends, or all at
+// once when a thread has used kMostStreams of them.
+// A capture may allocate nothing, and its graph keeps the addresses: captured
+// launches of a thread share one more, sized by its calls outside captures; what a
+// larger one replaces is kept (twice the size each time).
+struct StreamReducers {
+    static constexpr size_t kMostStreams = 16;
+    std::map<std::pair<int, unsigned long long>, Reducer> of;
+    std::map<int, std::vector<Reducer>> captured;  // per device, the last one in use
+    Reducer *for_capture(int dev, int grid, int ncol, bool grow) {
+        std::vector<Reducer> &v = captured[dev];
+        if (v.empty() || v.back().partial.bytes < Reducer::bytes(grid, ncol)) {
+            Reducer r;
+            if (!grow) {
+                fail(KMSD_ERUNTIME, "a captured sum needs scratch that a call outside the capture has sized");
+                return nullptr;
+            }
+            if (r.ensure(grid, v.empty() ? ncol : 2 * ncol)) return nullptr;
+            v.push_back(r);
+        }
+        return &v.back();
+    }
+    void release() {
+        // (frees may not break another thread's stream capture)
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        for (auto &kv : of) {
+            kv.second.partial.release();
+            kv.second.ticket.release();
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        of.clear();
+    }
+    ~StreamReducers() { release(); }
+};
+// nullptr on an error.
+Reducer *stream_reducer(cudaStream_t s, int grid, int ncol) {
+    static thread_local StreamReducers mine;
+    int dev = 0;
+    unsigned long long id = 0;  // (a stream's handle may come back for another one)
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaStreamIsCapturing(s, &capturing);
+    if (e == cudaSuccess && capturing == cudaStreamCaptureStatusActive) return mine.for_capture(dev, grid, ncol, false);
+    if (e == cudaSuccess) e = cudaStreamGetId(s, &id);
+    auto it = mine.of.find({dev, id});
+    if (e == cudaSuccess && it == mine.of.end()) {
+        if (mine.of.size() >= StreamReducers::kMostStreams) {
+            e = cudaDeviceSynchronize();
+            mine.release();
+        }
+        it = mine.of.emplace(std::make_pair(dev, id), Reducer{}).first;
+    }
+    if (e != cudaSuccess) {
+        cuda_fail(e, "the scratch of a stream");
+        return nullptr;
+    }
+    return it->second.ensure(grid, ncol) || !mine.for_capture(dev, grid, ncol, true) ? nullptr : &it->second;
+}
+
 template <class T, int MU, bool DOT>
 void launch_spmm(CsrView<T> A, const typename Unit<T>::vec *X, typename Unit<T>::vec *Y, int64_t n, RowMap mp,
-                 Reducer &red, double2 *dot, cudaStream_t s) {
+                 const Reducer &red, double2 *dot, cudaStream_t s) {
     const int grid = grid_for(n, mp);
     spmm_kernel<T, MU, DOT><<<grid, kThreads, reduce_smem(mp, Unit<T>::C), s>>>(A, X, Y, n, mp, red.part(),
                                                                                red.tick(), dot);
@@ -181,11 +243,15 @@ void launch_spmm(CsrView<T> A, const typename Unit<T>::vec *X, typename Unit<T>:
 template <class T>
 int spmm_any(CsrView<T> A, const typename Unit<T>::vec *X, typename Unit<T>::vec *Y, int64_t n, int U,
              cudaStream_t s, double2 *dot) {
-    static thread_local Reducer red;
     const RowMap mp = make_map(U, kThreads);
     const int mu = mu_for(mp);
     if (!mu) return fail(KMSD_EINVAL, "too many columns for one SpMM call");
-    if (red.ensure(grid_for(n, mp), U * Unit<T>::C)) return KMSD_ECUDA;
+    Reducer red;  // (without a dot product nothing is reduced)
+    if (dot) {
+        const Reducer *mine = stream_reducer(s, grid_for(n, mp), U * Unit<T>::C);
+        if (!mine) return KMSD_ECUDA;
+        red = *mine;
+    }
 #define KMSD_SPMM_CASE(M)                                                      \
     case M:                                                                    \
         if (dot) launch_spmm<T, M, true>(A, X, Y, n, mp, red, dot, s);         \
@@ -204,12 +270,16 @@ int spmm_any(CsrView<T> A, const typename Unit<T>::vec *X, typename Unit<T>::vec
 namespace kmsd {
 int spmm64(const kmsd_csr_s *A, const double2 *X, double2 *Y, int64_t b, cudaStream_t s, double2 *dot_out) {
     if (A->bsr_nb > 0) {
-        static thread_local Reducer red;
         const RowMap mp = make_map((int)b, kThreads);
         const int mu = mu_for(mp);
         if (!mu) return fail(KMSD_EINVAL, "too many columns for one SpMM call");
         const int grid = grid_for(A->bsr_nb, mp);
-        if (red.ensure(grid, (int)b)) return KMSD_ECUDA;
+        Reducer red;
+        if (dot_out) {
+            const Reducer *mine = stream_reducer(s, grid, (int)b);
+            if (!mine) return KMSD_ECUDA;
+            red = *mine;
+        }
         const size_t sm = reduce_smem(mp, 1);
         const BsrView<double> v = A->bsr64();
         const bool cplx = v.im != nullptr;
@@ -296,12 +366,13 @@ __global__ void __launch_bounds__(256) coldot_kernel(const typename Unit<T>::vec
 template <class T>
 int coldot_any(const typename Unit<T>::vec *x, const typename Unit<T>::vec *y, int64_t n, int U, double2 *out,
                cudaStream_t s) {
-    static thread_local Reducer red;
     const RowMap mp = make_map(U, kThreads);
     const int mu = mu_for(mp);
     if (!mu) return fail(KMSD_EINVAL, "too many columns for one reduction");
     const int grid = grid_for(n, mp);
-    if (red.ensure(grid, U * Unit<T>::C)) return KMSD_ECUDA;
+    const Reducer *mine = stream_reducer(s, grid, U * Unit<T>::C);
+    if (!mine) return KMSD_ECUDA;
+    const Reducer red = *mine;
     const size_t sm = reduce_smem(mp, Unit<T>::C);
     switch (mu) {
         case 1: coldot_kernel<T, 1><<<grid, kThreads, sm, s>>>(x, y, n, mp, red.part(), red.tick(), out); break;
@@ -513,7 +584,10 @@ int kmsd_check_finite(const void *x, int64_t count, int *finite, void *stream) {
     struct Flag {
         int *p = nullptr;
         ~Flag() {
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // (as StreamReducers::release)
+            cudaThreadExchangeStreamCaptureMode(&mode);
             if (p) cudaFreeHost(p);
+            cudaThreadExchangeStreamCaptureMode(&mode);
         }
     };
     static thread_local Flag flag;

@@ -124,6 +124,7 @@ int ring_slots();
 struct Reducer {
     DevBuf partial;
     DevBuf ticket;
+    static size_t bytes(int grid, int ncol) { return (size_t)tree_rows(grid) * ncol * sizeof(double2) + 64; }
     int ensure(int grid, int ncol, int copies = 1);
     double2 *part() const { return partial.as<double2>(); }
     Ticket *tick() const { return ticket.as<Ticket>(); }
