@@ -340,13 +340,12 @@ template <class T> double step_cycles(int64_t rows, int cols, int width, bool do
 namespace kmsd {
 
 size_t cluster_smem_limit() {
-    static const size_t limit = [] {
-        int dev = 0, optin = 0;
-        cudaGetDevice(&dev);
+    static PerDevice<size_t> limit;
+    return limit.get([](int dev) {
+        int optin = 0;
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         return (size_t)optin - 1024;
-    }();
-    return limit;
+    });
 }
 
 void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, int ctas, int size, int threads, size_t smem) {
@@ -362,9 +361,9 @@ void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, int ctas, 
 
 int active_clusters(const void *kernel, int size, int threads, size_t smem) {
     static std::mutex lock;
-    static std::map<std::tuple<const void *, int, int, size_t>, int> cache;
+    static std::map<std::tuple<int, const void *, int, int, size_t>, int> cache;
     std::lock_guard<std::mutex> guard(lock);
-    const auto key = std::make_tuple(kernel, size, threads, smem);
+    const auto key = std::make_tuple(current_device(), kernel, size, threads, smem);
     auto it = cache.find(key);
     if (it != cache.end()) return it->second;
     int n = 0;
@@ -387,8 +386,8 @@ int cluster_plan(int64_t n, int width, int64_t b, bool doubling, ClusterPlan *ou
     *out = ClusterPlan{};
     if (width < 1 || width > kClusterWidth) return KMSD_OK;
     static std::mutex lock;
-    static std::map<std::tuple<int64_t, int, int64_t, bool>, ClusterPlan> cache;
-    const auto key = std::make_tuple(n, width, b, doubling);
+    static std::map<std::tuple<int, int64_t, int, int64_t, bool>, ClusterPlan> cache;
+    const auto key = std::make_tuple(current_device(), n, width, b, doubling);
     {
         std::lock_guard<std::mutex> guard(lock);
         const auto it = cache.find(key);

@@ -357,8 +357,8 @@ template <class T> int find_plan(int what, int64_t n, int width, int64_t nb, Clu
     *out = ClusterPlan{};
     if (width < 1 || width > kClusterWidth) return KMSD_OK;
     static std::mutex lock;
-    static std::map<std::tuple<int, int64_t, int, int64_t>, ClusterPlan> cache;
-    const auto key = std::make_tuple(what, n, width, nb);
+    static std::map<std::tuple<int, int, int64_t, int, int64_t>, ClusterPlan> cache;
+    const auto key = std::make_tuple(current_device(), what, n, width, nb);
     const int planes = what == kChain ? 2 : what == kPsi ? 3 : 6, blocks = what == kPsiPhi ? 2 : 1;
     {
         std::lock_guard<std::mutex> guard(lock);

@@ -249,9 +249,11 @@ int corr_ring(const double2 *ring, int64_t n, int nb, const double2 *cov, int k1
     const int64_t rows_per = (n + nchunks - 1) / nchunks;
     nchunks = (int)((n + rows_per - 1) / rows_per);
     if (partial.ensure((size_t)nchunks * kRing * k1 * nb * sizeof(double2))) return KMSD_ECUDA;
-    static const cudaError_t attr = cudaFuncSetAttribute((const void *)corr_partial_kernel,
-                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    KMSD_CUDA(attr);
+    static PerDevice<cudaError_t> attr;
+    KMSD_CUDA(attr.get([](int) {
+        return cudaFuncSetAttribute((const void *)corr_partial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    200 * 1024);
+    }));
     corr_partial_kernel<<<nchunks * ktiles, threads, smem, s>>>(ring, n * nb, cov, n, nb, nbp, k1, kw, j0, jn, rows_per,
                                                                 ktiles, rs, partial.as<double2>());
     count_launch();

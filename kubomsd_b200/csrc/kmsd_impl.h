@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -32,6 +33,26 @@ int cuda_fail(cudaError_t e, const char *what);
 inline bool settle() {
     const cudaError_t e = cudaStreamSynchronize(cudaStreamLegacy);
     return e != cudaSuccess && cuda_fail(e, "an upload");
+}
+
+// A value of each device, made when that device first needs it (kernel attributes
+// and occupancies belong to a device's context); for any number of threads.
+template <class V> struct PerDevice {
+    std::mutex lock;
+    std::map<int, V> of;
+    template <class Make> V get(Make &&make) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        std::lock_guard<std::mutex> guard(lock);
+        auto it = of.find(dev);
+        if (it == of.end()) it = of.emplace(dev, make(dev)).first;
+        return it->second;
+    }
+};
+inline int current_device() {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return dev;
 }
 
 // Grow-only device buffer.

@@ -1007,11 +1007,11 @@ const void *kernel_of(int form, int lcw, bool cplx) {
 }
 
 // Largest dynamic shared memory of a CTA, and the one-time attributes of the
-// kernels (per process, thread-safe).
+// kernels.
 int smem_limit() {
-    static const int limit = [] {
-        int dev = 0, optin = 0;
-        cudaGetDevice(&dev);
+    static PerDevice<int> limit;
+    return limit.get([](int dev) {
+        int optin = 0;
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         const int cap = optin - 1024;
         for (int form = kFormCluster; form <= kFormStream; ++form)
@@ -1022,17 +1022,18 @@ int smem_limit() {
                     if (form == kFormCluster) cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
                 }
         return cap;
-    }();
-    return limit;
+    });
 }
 
 // Whether 16 CTAs with the largest shared memory fit one cluster on this device.
 bool cluster_fits() {
-    static const bool fits = [] {
+    static PerDevice<bool> fits;
+    const int smem = smem_limit();
+    return fits.get([smem](int) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(kClusterCtas);
         cfg.blockDim = dim3(kResThreads);
-        cfg.dynamicSmemBytes = smem_limit();
+        cfg.dynamicSmemBytes = smem;
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = kClusterCtas;
@@ -1045,8 +1046,7 @@ bool cluster_fits() {
             return false;
         }
         return n > 0;
-    }();
-    return fits;
+    });
 }
 
 // The block columns that each CTA's rows touch (its halo), sorted, with its own
