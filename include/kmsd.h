@@ -416,7 +416,8 @@ int kmsd_batch_moments(kmsd_batch bt, const void *b_in, double *mu, int64_t b,
 int kmsd_batch_set_tile_rows(kmsd_batch bt, int64_t tile_rows);
 
 /* Autotuner: times the tile sizes 512..8192 rows on this call's shape and
- * keeps the fastest (written to *chosen_tile_rows). */
+ * keeps the fastest (written to *chosen_tile_rows).  A call that runs as one
+ * launch has no tiles: one call, and the current size is kept. */
 int kmsd_batch_tune(kmsd_batch bt, const void *b_in, double *mu, int64_t b,
                     int64_t length, const double *center, const double *half,
                     int flags, int64_t *chosen_tile_rows, void *stream);

@@ -129,7 +129,8 @@ class B200Batch:
     def tune(self, B, length, centers, halves, doubling=True):
         """Autotunes the row-tile size and the vector-block width: for each
         width (all columns, half, a quarter; even widths in the mixed form)
-        the library sweeps the tile sizes, then whole calls with that width
+        the library sweeps the tile sizes (calls that run as one launch have no
+        tiles and keep the current size), then whole calls with that width
         and its best tile are timed.  Keeps the fastest pair; returns the tile
         rows (the width is in `col_block`)."""
         torch = _torch()

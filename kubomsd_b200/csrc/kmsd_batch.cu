@@ -234,6 +234,7 @@ struct kmsd_batch_s {
     int width = 0;  // entries of the longest row, 0: an instance has complex entries
     std::map<std::pair<int64_t, bool>, Clusters> clusters;
     std::vector<ClusterSystem> last_systems;
+    bool one_launch = false;  // the last orthogonal call took that path
     DevBuf systems, sums;
     int64_t general_kernels = 0;  // host-side kernels recorded in the nonorthogonal graph
 };
@@ -510,9 +511,8 @@ int run_clusters(kmsd_batch_s *bt, const double2 *B, double *mu, int64_t b, int6
 template <class T>
 int run_batch(kmsd_batch_s *bt, const double2 *B, double *mu, int64_t b, int64_t length, bool doubling,
               cudaStream_t s, bool use_graph) {
-    bool done = false;
-    if (int rc = run_clusters<T>(bt, B, mu, b, length, doubling, s, &done)) return rc;
-    if (done) return KMSD_OK;
+    if (int rc = run_clusters<T>(bt, B, mu, b, length, doubling, s, &bt->one_launch)) return rc;
+    if (bt->one_launch) return KMSD_OK;
     constexpr int C = Unit<T>::C;
     const int U = (int)((b + C - 1) / C);
     const RowMap mp = make_map(U, kThreads);
@@ -838,6 +838,7 @@ int kmsd_batch_tune(kmsd_batch bt, const void *b_in, double *mu, int64_t b, int6
         int rc = build_tiles(bt, rows);
         if (!rc) rc = batch_call(bt, b_in, mu, b, length, center, half, flags, s, false);  // warm
         if (rc) return rc;
+        if (!bt->gm && bt->one_launch) break;  // no tiles in it: the size stays
         KMSD_CUDA(cudaEventRecord(e0, s));
         rc = batch_call(bt, b_in, mu, b, length, center, half, flags, s, false);
         if (rc) return rc;
