@@ -492,8 +492,9 @@ int run_clusters(kmsd_batch_s *bt, const double2 *B, double *mu, int64_t b, int6
     for (int64_t i = 0; i < bt->ninst; ++i)
         sys[i] = ClusterSystem{bt->row_off[i], bt->row_off[i + 1] - bt->row_off[i], bt->last_center[i], bt->last_half[i],
                                mu + (size_t)i * length * b};
-    if (bt->systems.ensure(sys.size() * sizeof(ClusterSystem)) || bt->sums.ensure(cluster_scratch(cl.plan, length, doubling)))
-        return KMSD_ECUDA;
+    // (the sums grow with the number of moments; the step kernels need none)
+    if (bt->systems.ensure(sys.size() * sizeof(ClusterSystem))) return KMSD_ECUDA;
+    if (bt->sums.try_ensure(cluster_scratch(cl.plan, length, doubling))) return KMSD_OK;
     if (bt->last_systems.size() != sys.size() ||
         std::memcmp(bt->last_systems.data(), sys.data(), sys.size() * sizeof(ClusterSystem)) != 0) {
         KMSD_CUDA(cudaMemcpyAsync(bt->systems.p, sys.data(), sys.size() * sizeof(ClusterSystem), cudaMemcpyHostToDevice, s));

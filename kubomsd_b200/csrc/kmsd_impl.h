@@ -60,6 +60,13 @@ struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
     int ensure(size_t want);
+    // As ensure, for a path that another one can stand in for: a failure leaves no
+    // CUDA error behind for the next check to find.
+    int try_ensure(size_t want) {
+        const int rc = ensure(want);
+        if (rc) cudaGetLastError();
+        return rc;
+    }
     void release();
     template <class X> X *as() const { return static_cast<X *>(p); }
 };

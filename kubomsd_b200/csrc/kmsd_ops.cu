@@ -336,7 +336,8 @@ int moments_small(E *e, const double2 *B, double *mu, int64_t b, int64_t len, do
     ClusterPlan pl;
     int rc = cluster_plan<T>(e->H->n, e->H->row_max, b, doubling, &pl);
     if (rc || !pl.size) return rc;
-    if (e->cluster.ensure(cluster_scratch(pl, len, doubling))) return KMSD_ECUDA;
+    // (its sums grow with the number of moments; the step kernels need none)
+    if (e->cluster.try_ensure(cluster_scratch(pl, len, doubling))) return KMSD_OK;
     if (std::is_same<T, float>::value && e->H->ensure_f32()) return KMSD_ECUDA;
     const ClusterSystem one{0, e->H->n, center, half, mu};
     rc = cluster_moments<T>(pl, view_of<T>(e->H), e->H->row_max, B, b, len, doubling, nullptr, nullptr, one,
@@ -814,7 +815,8 @@ bool imaginary_velocity(E *e, int x) {
         }
     }
     const std::vector<float> im32(im.begin(), im.end());
-    if (e->vcsr64[x].ensure(im.size() * sizeof(double)) || e->vcsr32[x].ensure(im32.size() * sizeof(float))) return false;
+    if (e->vcsr64[x].try_ensure(im.size() * sizeof(double)) || e->vcsr32[x].try_ensure(im32.size() * sizeof(float)))
+        return false;
     if (cudaMemcpy(e->vcsr64[x].p, im.data(), im.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(e->vcsr32[x].p, im32.data(), im32.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess || settle())
         return false;
