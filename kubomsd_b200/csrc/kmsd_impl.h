@@ -188,7 +188,7 @@ struct kmsd_metric_s {
     struct Halo {
         kmsd::DevBuf mem;
         int *off = nullptr, *list = nullptr, *local = nullptr, *self = nullptr;
-        int own = 0, blocks = 0, most = 0;  // of the largest CTA share
+        int most = 0;  // block columns of the largest one
     };
     std::map<int, Halo> halos;
     kmsd::Reducer red;

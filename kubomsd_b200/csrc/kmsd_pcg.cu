@@ -1049,6 +1049,17 @@ bool cluster_fits() {
     });
 }
 
+// Block rows and S blocks of the largest CTA share.
+void largest_share(const kmsd_csr_s *S, int ctas, int *own, int *blocks) {
+    const int64_t nbr = S->bsr_nb;
+    *own = *blocks = 0;
+    for (int c = 0; c < ctas; ++c) {
+        const int64_t i0 = nbr * c / ctas, i1 = nbr * (c + 1) / ctas;
+        *own = std::max(*own, (int)(i1 - i0));
+        *blocks = std::max(*blocks, S->bsr_ptr_host[i1] - S->bsr_ptr_host[i0]);
+    }
+}
+
 // The block columns that each CTA's rows touch (its halo), sorted, with its own
 // block rows among them, and every block's place in its CTA's list.
 int halo_of(kmsd_metric_s *M, int ctas, kmsd_metric_s::Halo **out) {
@@ -1073,8 +1084,6 @@ int halo_of(kmsd_metric_s *M, int ctas, kmsd_metric_s::Halo **out) {
         for (int64_t i = i0; i < i1; ++i) self[i] = place[i];
         list.insert(list.end(), cols.begin(), cols.end());
         off[c + 1] = (int)list.size();
-        h.own = std::max(h.own, (int)(i1 - i0));
-        h.blocks = std::max(h.blocks, k1 - k0);
         h.most = std::max(h.most, (int)cols.size());
     }
     const size_t n[4] = {off.size(), list.size(), local.size(), self.size()};
@@ -1114,18 +1123,24 @@ int resident_plan(kmsd_metric_s *M, int64_t b, ResidentPlan *out) {
     // every thread owns one (block row, column); the blocks of a row are split
     // over as many lanes as are left
     auto resident = [&](int form, int ctas) -> int {
-        kmsd_metric_s::Halo *h;
         if ((1 << full) < b || S->bsr_nb > (int64_t)ctas * (kResThreads >> full)) return KMSD_OK;
+        largest_share(S, ctas, &pl.own, &pl.blocks);
+        if (pl.own > kResThreads >> full) return KMSD_OK;
+        auto smem = [&](int most) {
+            return state_bytes(kResThreads, 1 << full, form == kFormCluster) +
+                   slice_bytes(pl.own, pl.blocks, cplx, pre_d, most, kResidentUnits) + ((size_t)most << (full + 6));
+        };
+        // a halo holds the CTA's own block rows; its lists are made where it may fit
+        if (smem(pl.own) > limit) return KMSD_OK;
+        kmsd_metric_s::Halo *h;
         if (int rc = halo_of(M, ctas, &h)) return rc;
-        const bool cl = form == kFormCluster;
-        pl.smem = state_bytes(kResThreads, 1 << full, cl) + slice_bytes(h->own, h->blocks, cplx, pre_d, h->most, kResidentUnits) +
-                  ((size_t)h->most << (full + 6));
-        if (pl.smem > limit || h->own > kResThreads >> full) return KMSD_OK;
+        pl.smem = smem(h->most);
+        if (pl.smem > limit) return KMSD_OK;
         pl.form = form;
         pl.ctas = ctas;
         pl.threads = kResThreads;
         pl.lks = 0;
-        while (full + pl.lks < 5 && pl.lks < 3 && h->own <= kResThreads >> (full + pl.lks + 1)) ++pl.lks;
+        while (full + pl.lks < 5 && pl.lks < 3 && pl.own <= kResThreads >> (full + pl.lks + 1)) ++pl.lks;
         pl.halo = h;
         return KMSD_OK;
     };
@@ -1134,16 +1149,14 @@ int resident_plan(kmsd_metric_s *M, int64_t b, ResidentPlan *out) {
     if (!rc && !pl.form) rc = resident(kFormGrid, sms);
     if (rc) return rc;
     if (!pl.form) {
-        kmsd_metric_s::Halo *h;
-        if ((rc = halo_of(M, sms, &h))) return rc;
+        largest_share(S, sms, &pl.own, &pl.blocks);
         pl.nch = (int)((b + (1 << full) - 1) >> full);
-        pl.smem = state_bytes(kStreamThreads, pl.nch << full, false) + slice_bytes(h->own, h->blocks, cplx, pre_d, 0, kStreamUnits);
+        pl.smem = state_bytes(kStreamThreads, pl.nch << full, false) + slice_bytes(pl.own, pl.blocks, cplx, pre_d, 0, kStreamUnits);
         if (pl.smem <= limit) {
             pl.form = kFormStream;
             pl.ctas = sms;
             pl.threads = kStreamThreads;
             pl.lks = 0;
-            pl.halo = h;
         }
     }
     if (!pl.form) return KMSD_OK;
@@ -1176,10 +1189,13 @@ int resident_solve(kmsd_metric_s *M, const ResidentPlan &pl, const double2 *B, d
     a.diag = M->diag;
     a.minv = M->nblocks > 0 ? M->factors : nullptr;
     a.minv_real = M->inv_real;
-    a.halo_off = pl.halo->off;
-    a.halo = pl.halo->list;
-    a.local = pl.halo->local;
-    a.self = pl.halo->self;
+    if (pl.halo) {
+        a.halo_off = pl.halo->off;
+        a.halo = pl.halo->list;
+        a.local = pl.halo->local;
+        a.self = pl.halo->self;
+        a.halos = pl.halo->most;
+    }
     a.c = col_ptr(M->cols.p, b);
     a.cnt = M->dcount.as<Counters>();
     a.rtol = rtol;
@@ -1195,9 +1211,8 @@ int resident_solve(kmsd_metric_s *M, const ResidentPlan &pl, const double2 *B, d
     a.lcw = pl.lcw;
     a.lks = pl.lks;
     a.nch = pl.nch;
-    a.own = pl.halo->own;
-    a.blocks = pl.halo->blocks;
-    a.halos = pl.halo->most;
+    a.own = pl.own;
+    a.blocks = pl.blocks;
     KMSD_CUDA(cudaMemsetAsync(a.bar, 0, 2 * sizeof(unsigned), s));  // (not the packets' sequence base)
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(pl.ctas);

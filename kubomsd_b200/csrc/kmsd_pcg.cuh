@@ -56,7 +56,8 @@ struct ResidentPlan {
     int ctas = 0, threads = 0;
     size_t smem = 0;
     int lcw = 0, lks = 0, nch = 1;  // log2 of a chunk's columns and of the lanes that split a block row; chunks
-    const kmsd_metric_s::Halo *halo = nullptr;
+    int own = 0, blocks = 0;                     // block rows and S blocks of the largest CTA share
+    const kmsd_metric_s::Halo *halo = nullptr;  // of the forms that stage it
 };
 int resident_plan(kmsd_metric_s *M, int64_t b, ResidentPlan *out);
 int resident_solve(kmsd_metric_s *M, const ResidentPlan &pl, const double2 *B, double2 *Y, int64_t b, double rtol,

@@ -39,7 +39,7 @@ def test_moments_without_room_for_the_cluster_sums(cuda, batch):
 
     def make(m):
         if batch:
-            return B200Batch([m.H], precision="fp64")
+            return B200Batch([m.H], precision="fp64", tile_rows=64)
         return engine(m.H, m.S)[1]
 
     def run(obj, x, length):
