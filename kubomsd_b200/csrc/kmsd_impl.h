@@ -191,6 +191,7 @@ struct kmsd_metric_s {
         int most = 0;  // block columns of the largest one
     };
     std::map<int, Halo> halos;
+    int64_t no_room = INT64_MAX;  // (padded) columns for which its memory could not be had
     kmsd::Reducer red;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     // counters (host side, plus device counters folded in on read)

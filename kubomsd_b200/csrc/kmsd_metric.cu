@@ -1020,6 +1020,7 @@ int kmsd_metric_s::ensure(int64_t b, int64_t state_cols) {
     if (cols.ensure(col_bytes(std::max(b, state_cols)))) return KMSD_ECUDA;
     if (b <= wb && q.p) return KMSD_OK;
     const size_t bytes = (size_t)n * b * sizeof(double2);
+    wb = 0;  // until all of them are there: a failure leaves some without memory
     for (DevBuf *d : {&q, &y, &r, &z, &p, &sp, &t})
         if (d->ensure(bytes)) return KMSD_ECUDA;
     if (!dcount.p) {

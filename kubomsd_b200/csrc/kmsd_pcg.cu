@@ -1061,7 +1061,8 @@ void largest_share(const kmsd_csr_s *S, int ctas, int *own, int *blocks) {
 }
 
 // The block columns that each CTA's rows touch (its halo), sorted, with its own
-// block rows among them, and every block's place in its CTA's list.
+// block rows among them, and every block's place in its CTA's list; nullptr where
+// there is no memory for them.
 int halo_of(kmsd_metric_s *M, int ctas, kmsd_metric_s::Halo **out) {
     auto it = M->halos.find(ctas);
     if (it != M->halos.end()) {
@@ -1088,7 +1089,10 @@ int halo_of(kmsd_metric_s *M, int ctas, kmsd_metric_s::Halo **out) {
     }
     const size_t n[4] = {off.size(), list.size(), local.size(), self.size()};
     const std::vector<int> *src[4] = {&off, &list, &local, &self};
-    if (h.mem.ensure((n[0] + n[1] + n[2] + n[3]) * sizeof(int))) return KMSD_ECUDA;
+    if (h.mem.try_ensure((n[0] + n[1] + n[2] + n[3]) * sizeof(int))) {
+        *out = nullptr;
+        return KMSD_OK;
+    }
     int *d = h.mem.as<int>();
     int **dst[4] = {&h.off, &h.list, &h.local, &h.self};
     for (int i = 0; i < 4; ++i) {
@@ -1134,6 +1138,7 @@ int resident_plan(kmsd_metric_s *M, int64_t b, ResidentPlan *out) {
         if (smem(pl.own) > limit) return KMSD_OK;
         kmsd_metric_s::Halo *h;
         if (int rc = halo_of(M, ctas, &h)) return rc;
+        if (!h) return KMSD_OK;
         pl.smem = smem(h->most);
         if (pl.smem > limit) return KMSD_OK;
         pl.form = form;
@@ -1162,12 +1167,23 @@ int resident_plan(kmsd_metric_s *M, int64_t b, ResidentPlan *out) {
     if (!pl.form) return KMSD_OK;
     const size_t cols = (size_t)pl.nch << pl.lcw;
     const size_t bytes = 256 + 4 * cols * (pl.ctas + 1) * sizeof(uint4);
+    // The vectors are padded to whole chunks, to less than twice b columns from 5 on.
+    // Where that does not fit, the launch sequence runs in b columns.
+    if ((int64_t)cols >= M->no_room) return KMSD_OK;
     if (M->resident.bytes < bytes) {
-        if (M->resident.ensure(bytes)) return KMSD_ECUDA;
+        if (M->resident.try_ensure(bytes)) {
+            M->no_room = (int64_t)cols;
+            return KMSD_OK;
+        }
         KMSD_CUDA(cudaMemset(M->resident.p, 0, bytes));
         if (settle()) return KMSD_ECUDA;
     }
-    if (M->ensure((int64_t)cols, b)) return KMSD_ECUDA;
+    if (M->ensure((int64_t)cols, b)) {
+        cudaGetLastError();
+        M->no_room = (int64_t)cols;
+        for (DevBuf *d : {&M->q, &M->y, &M->r, &M->z, &M->p, &M->sp, &M->t}) d->release();
+        return M->ensure(b, b) ? KMSD_ECUDA : KMSD_OK;
+    }
     *out = pl;
     return KMSD_OK;
 }

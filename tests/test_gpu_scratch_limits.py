@@ -63,3 +63,42 @@ def test_moments_without_room_for_the_cluster_sums(cuda, batch):
     assert rc == 0, _abi.last_error(obj.lib)
     assert obj.lib.kmsd_kernel_launches() - before >= M // 2  # a launch per step
     assert float((got - want.cpu()).abs().max()) <= 1e-9 * float(want.abs().max())
+
+
+def test_solve_without_room_for_padded_vectors(cuda):
+    """33 columns run as 64 in one launch: seven vectors of 32,000 rows, 229 MB instead
+    of 118.  The launch sequence solves them in what is left, on the same handle later
+    too."""
+    import numpy as np
+    from kubomsd_b200 import lattices
+    from tests.gpu_util import engine
+    torch = cuda
+    m = lattices.diamond_sp3(cells=10, scale_hint=.24)
+    S = m.S.tocsr()
+    blocks = [(i, j, np.linalg.cholesky(S[i:j, i:j].toarray())) for i, j in m.atom_slices]
+    roomy, eng, _ = engine(m.H, S, blocks=blocks)
+    cfg = roomy._create[2]
+    tight, other = roomy.replica(), roomy.replica()
+    B = torch.randn((S.shape[0], 33), dtype=torch.complex128, device="cuda")
+    lib = roomy.lib
+
+    def solve(metric):
+        before = lib.kmsd_kernel_launches()
+        x, report = metric.solve(B, cfg)
+        assert report.converged.all()
+        return x, lib.kmsd_kernel_launches() - before
+
+    want, launches = solve(roomy)
+    assert launches <= 3
+    other.set_storage("mixed")
+    solve(other)  # the kernels of the launch sequence are loaded
+    torch.cuda.synchronize()
+    with _left(torch, 190 << 20):
+        got, launches = solve(tight)
+        assert launches > 100
+        again, _ = solve(tight)
+        tight.solve(B[:, :4].contiguous(), cfg)
+    # both meet |b - S x| <= 1e-10 |b|, kappa(S) is 50
+    bound = 1.01 * 2 * 50 * 1e-10
+    assert float(((got - want).norm(dim=0) / want.norm(dim=0)).max()) <= bound
+    assert torch.equal(got, again)
