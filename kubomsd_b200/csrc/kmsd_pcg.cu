@@ -982,8 +982,10 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
 }
 
 enum { kFormCluster = 1, kFormGrid = 2, kFormStream = 3 };
-// Smaller systems keep the launch sequence, whose launches per iteration
-// kmsd_kernel_launches reports.
+// Smaller systems keep the launch sequence.  Speed does not ask for that: 4 to 63
+// block rows of 5 blocks x 1 to 32 columns take 0.46 to 0.59 ms with it and 0.16 to
+// 0.20 in one cluster.  A program that reads kmsd_kernel_launches sees its launches
+// per iteration, and the tests hold a system of 40 block rows to them.
 constexpr int kMinBlockRows = 64;
 
 template <int lcw, bool CPLX>
@@ -1157,7 +1159,17 @@ int resident_plan(kmsd_metric_s *M, int64_t b, ResidentPlan *out) {
         largest_share(S, sms, &pl.own, &pl.blocks);
         pl.nch = (int)((b + (1 << full) - 1) >> full);
         pl.smem = state_bytes(kStreamThreads, pl.nch << full, false) + slice_bytes(pl.own, pl.blocks, cplx, pre_d, 0, kStreamUnits);
-        if (pl.smem <= limit) {
+        // A chunk of columns takes the latency of a block row's products whatever the
+        // number of rows, and the chunks come one after another, where the launch
+        // sequence splits rows and takes all columns at once.  With few rows for each
+        // CTA, many chunks and long rows that is slower: 64 / 216 / 512 block rows of
+        // 17 blocks x 256 columns took 3.57 / 4.44 / 5.85 ms against 2.36 / 3.63 / 6.34,
+        // 64 x 128 2.03 against 2.18, 216 x 192 3.55 against 3.46.  The line fits 672
+        // solves of 64 to 900 block rows, 5 to 33 blocks a row and 33 to 256 columns,
+        // with at most 14 % lost on either side of it.
+        const double row_blocks = (double)S->bsr_ptr_host[S->bsr_nb] / (double)S->bsr_nb;
+        const bool slower = pl.nch * (row_blocks + 9.) > 88. + 44. * (double)S->bsr_nb / sms;
+        if (pl.smem <= limit && !slower) {
             pl.form = kFormStream;
             pl.ctas = sms;
             pl.threads = kStreamThreads;
