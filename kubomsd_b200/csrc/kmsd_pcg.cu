@@ -100,8 +100,10 @@ __host__ __device__ inline size_t slice_bytes(int own, int blocks, bool cplx, in
 }
 
 // Longest wait at a meeting of the CTAs, after which the solve gives up and the
-// call reports an error.
-constexpr unsigned long long kMeetNs = 2000000000ull;
+// call reports an error.  The CTAs of a cooperative launch begin as SMs come free,
+// so the first ones wait for what other streams still run; ten seconds leave room
+// for that.  The solves queued behind one that gave up do not wait again.
+constexpr unsigned long long kMeetNs = 10000000000ull;
 
 __device__ __forceinline__ unsigned long long clock_ns() {
     unsigned long long t;
@@ -303,12 +305,12 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
         }
     }
     unsigned base = 0;
-    bool gone = false;  // the others gave up before this CTA began
+    bool gone = false;  // the others gave up before this CTA began, or an earlier solve of the call did
     if constexpr (CL) {
         cluster_meet();  // every CTA of the cluster is running before its boxes are written
     } else {
         base = load_acquire(a.bar + 2);
-        gone = __syncthreads_or(load_acquire(a.bar + 1));
+        gone = __syncthreads_or(load_acquire(a.bar + 1) | load_acquire(reinterpret_cast<unsigned *>(a.status + 3)));
     }
 
     unsigned arrivals = 0, seq = base;
