@@ -454,7 +454,7 @@ def config_c2(threads, storage=("fp64", "mixed"), M=1024):
     ach = out[best]["bytes_per_pcg_iteration"] / (out[best]["us_per_pcg_iteration"] * 1e-6) / 1e9
     out["roofline"] = {"bound": "L2/latency: the PCG working set (seven 16 MB vector blocks, 17 MB of S) is "
                                 "L2-resident, so the HBM figure below is for information",
-                       "kernel": "PCG iteration (pcg_spmv + pcg_update + pcg_direction)", "achieved": ach,
+                       "kernel": "PCG iteration (pcg_resident_kernel; pcg_spmv + pcg_update + pcg_direction with complex64 storage)", "achieved": ach,
                        "peak": peak, "unit": "GB/s", "frac": ach / peak, "peak_source": peak_src_note(src),
                        "algorithmic_bytes_per_iteration": out[best]["bytes_per_pcg_iteration"]}
     ref = _ref_engine(m.H, S, threads, blocks=[(a0, b0, L) for a0, b0, L in blocks])
@@ -551,6 +551,9 @@ def config_c5(duration=3., rate=20., msd_fraction=.25):
                         + ", 8 slots, HBM budget 150 GB",
             "latency": latency_summary(res), "requests": len(res), "errors": len(srv.errors),
             "error_messages": sorted({msg for _, msg in srv.errors})[:5],
+            # solves whose acceptance missed by roundings and that went on from their true residual
+            "solve_continuations": sum(e.native.metric.stats().refinement_steps for m in models.values()
+                                       for e in list(m.pool.queue)),
             "jobs": {"dos": sum(r.kind == "dos" for r in res), "msd": sum(r.kind == "msd" for r in res)},
             "wall_s": wall, "requests_per_s": len(res) / wall, "offered_rate": rate,
             "slot_occupancy": busy / (8 * wall)}

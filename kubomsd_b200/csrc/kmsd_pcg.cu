@@ -25,21 +25,23 @@
 //            0.9 us behind global stores), leaves the other SMs to other
 //            streams, and puts its sums into the shared memory of all CTAs;
 //   grid     a cooperative launch of one CTA per SM, up to 56,832 pairs; sums
-//            travel as packets (below), about 2 us per reduction;
+//            travel as packets (below) and every reduction is a meeting too;
 //   stream   the same launch with the work vectors in memory (L2), any columns.
 // The first two copy the block columns that a CTA's rows touch (its halo) to
 // shared memory once per product and keep x, r, p and S p in registers; what
 // bounds them is the shared-memory reads of the product (see product()) and the
 // two meetings.  `stream` gathers z through L1; bound by that gather.
 //
-// Whole solves, block-Jacobi, rtol 1e-10, against the launch sequence:
-//   2,048 orbitals x 8 columns (cluster)    0.60 ms, 2.51 ms before
-//   6,912 x 13 (grid)                       0.95 ms, 3.19 ms
-//   32,000 x 32 (stream)                    4.6 ms,  8.2 ms
-//   55,296 x 16 (stream)                    4.5 ms,  9.4 ms
-// The grid form took 1.41 M cycles where the cluster form took 1.19 M on the
-// first, and 1.15 M against 1.07 M on 864 x 16; the stream form 2.74 M where the
-// grid form took 1.63 M on the second.
+// Whole solves through kmsd_metric_solve, block-Jacobi, rtol 1e-10, against the
+// launch sequence on the same box (about 72 iterations each):
+//   2,048 orbitals x 8 columns (cluster)    0.71 ms, 3.00 ms before
+//   6,912 x 12 (grid)                       0.84 ms, 3.09 ms
+//   32,000 x 32 (stream)                    4.58 ms, 8.24 ms
+//   55,296 x 16 (stream)                    4.54 ms, 9.40 ms
+// The cluster form against the grid form: 0.48 and 0.58 ms on 864 x 4, 0.70 and
+// 0.72 on 2,048 x 8, 0.63 and 0.61 on 864 x 16, where it takes a ninth of the SMs.
+// The grid form against the stream form: 0.84 and 1.23 on 6,912 x 12, 1.53 and 2.17
+// on 16,384 x 8.
 #include <algorithm>
 #include <cfloat>
 #include <climits>
@@ -79,9 +81,10 @@ struct ResArgs {
 constexpr int kStateDoubles = 8, kStateInts = 4;
 constexpr int kAhead = 1;
 // Continuations of a solve at most, and how far above its threshold a column's true
-// residual may be for one.
+// residual may be for one: where roundings move it by more than the threshold, the
+// tolerance is not attainable.
 constexpr int kMostRedos = 4;
-constexpr double kRedoWithin = 1. + 1. / 1024.;
+constexpr double kRedoWithin = 2.;
 constexpr int kResThreads = 384, kStreamThreads = 512, kClusterCtas = 16;
 // 16-byte units from one S block in shared memory to the next: in the resident
 // forms one more than its 8, so that lanes on neighbouring blocks read from
@@ -819,10 +822,10 @@ __global__ void __launch_bounds__(RES ? kResThreads : kStreamThreads, 1) pcg_res
             if (accept) {
                 // Under the fixed policy a column leaves when the residual of its
                 // recurrence meets the threshold.  The true one is some roundings
-                // away, 1e-7 of the threshold at a tolerance of 1e-10 (5e-4 at
-                // 1e-13), and misses it in about one of 10^7 columns.  Such a column
-                // goes on from its true residual; one that is further off than
-                // roundings explain fails.
+                // away: at kappa(S) = 50 and a tolerance of 1e-10 by 1e-7 of the
+                // threshold, and about one of 10^7 columns misses it; both grow with
+                // kappa and with the tightness of the tolerance.  Such a column goes on
+                // from its true residual; one that is further off fails.
                 rnorm[j] = tn;
                 act = rst = !broken && !nonfinite && k < a.maxiter && redos < kMostRedos && tn > thr[j] &&
                             tn <= kRedoWithin * thr[j];

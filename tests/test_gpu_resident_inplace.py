@@ -45,9 +45,9 @@ def test_solution_over_its_right_hand_side(cuda, b):
 
 @pytest.mark.parametrize("b", [8, 32, 64])
 def test_columns_that_just_miss_go_on(cuda, b):
-    """A column above its threshold by at most 1/1024 goes on and converges, and the
-    solve is counted (kmsd_metric_stats.refinement_steps); one that is further off
-    fails the solve with its residual."""
+    """A column above its threshold by less than the threshold itself goes on and
+    converges, and the solve is counted (kmsd_metric_stats.refinement_steps); one that
+    is further off fails the solve with its residual."""
     from kubomsd_b200.errors import NumericalError
     torch = cuda
     rtol = 1e-14
@@ -63,7 +63,7 @@ def test_columns_that_just_miss_go_on(cuda, b):
             x, report = metric.solve(B, cfg)
         except NumericalError as exc:
             rel = np.array(exc.diagnostics["relative_residual"])
-            assert rel[~np.array(exc.diagnostics["converged"])].min() > rtol * (1 + 1 / 1024) * (1 - 1e-9)
+            assert rel[~np.array(exc.diagnostics["converged"])].min() > 2 * rtol * (1 - 1e-9)
             continue
         assert report.converged.all() and report.relative_residual.max() <= rtol * (1 + 1e-9)
         # formed once more, with roundings of about a hundredth of the threshold at most
