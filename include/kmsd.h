@@ -152,8 +152,8 @@ int kmsd_metric_set_residual_policy(kmsd_metric m, int policy, int interval,
  * max(rtol*||q||, atol/safe), curvature-breakdown test, true-residual refresh
  * every `interval` iterations, final true-residual acceptance and
  * representability checks (Metric::solve, cpp/native.cpp:313-452).
- * Synchronises the stream once to read the per-column status.  On failure
- * returns KMSD_EMETRIC with the reference's message and fills `report`
+ * y_out may be b_in.  Synchronises the stream once to read the per-column
+ * status.  On failure returns KMSD_EMETRIC with the reference's message and fills `report`
  * (which may be NULL when not wanted). */
 int kmsd_metric_solve(kmsd_metric m, const void *b_in, void *y_out, int64_t b,
                       double rtol, double atol, int maxiter,

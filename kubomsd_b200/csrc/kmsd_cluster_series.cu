@@ -1,10 +1,9 @@
 // The Bessel series and stored Chebyshev chains of small orthogonal-basis
 // operators in one launch.
 //
-// Series: the
-// propagation sum_k c_k T_k(A) of psi columns, alone or with the phi block of one
-// direction whose velocity is purely imaginary (the lattice velocities i H_ij
-// dx_ij / hbar).
+// Series: the propagation sum_k c_k T_k(A) of psi columns, alone or with the phi
+// block of one direction whose velocity is purely imaginary (the lattice velocities
+// i H_ij dx_ij / hbar).
 //
 // As kmsd_cluster.cu: a thread-block cluster takes a few psi columns and their phi
 // columns through all terms, with T_k, T_{k-1} and the accumulator in shared
