@@ -403,7 +403,18 @@ namespace kmsd {
 template <class T> int series_plan(int64_t n, int width, int64_t nb, bool phi, ClusterPlan *out) {
     return find_plan<T>(phi ? kPsiPhi : kPsi, n, width, nb, out);
 }
+// A chain stores n x b complex128 values every step, from the few clusters that run
+// at once; the step kernels store them from all SMs.  16 steps of 14,000 sites x 32
+// columns of five entries a row take 0.22 ms against 0.28 in complex128 and 0.21
+// against 0.28 in complex64, x 64 0.39 against 0.38 and 0.38 against 0.36, x 128 0.73
+// against 0.63 and 0.69 against 0.53; with rows of more than five complex128 entries
+// 4,096 x 64 takes 0.24 against 0.27 and x 128 0.39 against 0.32.
 template <class T> int chain_plan(int64_t n, int width, int64_t b, ClusterPlan *out) {
+    const int64_t most = sizeof(T) == 8 && width > 5 ? 500000 : 850000;
+    if (n * b > most) {
+        *out = ClusterPlan{};
+        return KMSD_OK;
+    }
     return find_plan<T>(kChain, n, width, b, out);
 }
 
