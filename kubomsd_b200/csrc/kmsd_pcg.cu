@@ -33,7 +33,7 @@
 // two meetings.  `stream` gathers z through L1; bound by that gather.
 //
 // Whole solves through kmsd_metric_solve, block-Jacobi, rtol 1e-10, against the
-// launch sequence on the same box (about 72 iterations each):
+// launch sequence in turn with it (about 72 iterations each):
 //   2,048 orbitals x 8 columns (cluster)    0.71 ms, 3.00 ms before
 //   6,912 x 12 (grid)                       0.84 ms, 3.09 ms
 //   32,000 x 32 (stream)                    4.58 ms, 8.24 ms
