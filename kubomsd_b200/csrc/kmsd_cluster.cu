@@ -17,11 +17,12 @@
 // fused multiply-adds, store) and the meeting, 0.8-1 us a step; for many, the
 // shared-memory traffic, (W + 3) elements per row and column.  A cluster of up to
 // 16 CTAs whose threads own up to 4 rows covers about 30,000 rows.  M = 512
-// direct moments of 4,096 sites x 8 complex128 columns took 0.52 ms against 4.33
+// direct moments of 4,096 sites x 8 complex128 columns take 0.46 ms against 4.33
 // with a launch per step; 511 of 16,129 x 31 complex64 by the product identity
-// 0.81 ms against 5.39; 256 of 24 lattices of 576 to 25,600 sites x 16 complex64
-// in one launch 2.28 ms against 9.10.  Within its reach it was the faster one everywhere: from
-// 512 to 30,720 rows and 1 to 256 columns by 1.5 (28,900 x 256) to 10 times.
+// 0.75 ms against 5.38; 256 of 24 lattices of 576 to 25,600 sites x 16 complex64
+// in one launch 2.29 ms against 9.00.  Within its reach it is the faster one
+// everywhere: from 1,000 to 36,000 rows of 3 to 7 entries and 2 to 128 columns by 1.3
+// (9,000 rows of 7 x 128, direct: 1.22 ms against 1.54) to 17 times.
 //
 // The arithmetic of an element is that of cheb_step_kernel, entry by entry, so
 // complex64 vectors come out bit-identical; the FP64 sums are taken in another
